@@ -194,12 +194,6 @@ __device__ __forceinline__ bool quad_of(const int n[3], Quad& q) {
     return q.z0 < n[2] && q.y < n[1];
 }
 
-// The operator at the four cells of a quad, rearranged so that a cell needs one division.  With
-// q = sum_a h_a^2 p_a^2 (so g = beta / q) and P = sum_a p_a^2:
-//   U = sum_a (v+a + v-a) / h_a^2
-//   W = sum_a p_a^2 (v+a + v-a) + 1/2 sum_{a<b} p_a p_b e_ab [+ sum_a p_a (v+a - v-a), local]
-//   S(v) = U + g W,   2 sum_a G_a = 2 (sum_a 1/h_a^2 + g P).
-// x and y are fixed for the thread, so the p_0, p_1 terms are computed once for its four cells.
 // The nine columns a quad's operator reads: the centre and the four axis neighbours at z0 - 1 .. z0 + 4,
 // the four (x +- 1, y +- 1) edge columns at z0 .. z0 + 3.
 template <typename V> struct QuadCols {
@@ -241,141 +235,125 @@ __device__ __forceinline__ void quad_load(const V* __restrict__ v, const Stencil
     load4(v + xp + ym + q.z0, Q.PM);
 }
 
-// The operator at the four cells of a quad (x, y, z0 .. z0 + 3), rearranged so that a cell needs one
-// division.  With q = sum_a h_a^2 p_a^2 (so g = beta / q) and P = sum_a p_a^2:
-//   U = sum_a (v+a + v-a) / h_a^2
-//   W = sum_a p_a^2 (v+a + v-a) + 1/2 sum_{a<b} p_a p_b e_ab [+ sum_a p_a (v+a - v-a), local]
-//   S(v) = U + g W,   2 sum_a G_a = 2 (sum_a 1/h_a^2 + g P).
-// x and y are fixed for the thread, so the p_0, p_1 terms are computed once for its four cells.  Every
-// quad kernel (one sweep from global memory, two sweeps from shared memory) evaluates this function.
-template <typename A, typename V, typename S, int MODE>
-__device__ __forceinline__ void quad_compute(const QuadCols<V>& Q, const Stencil<S>& s, int x, int y, int z0,
-                                             A (&U)[4], A (&W)[4], A (&qq)[4], A (&P)[4]) {
+}  // namespace prc
+
+#include "mg_march.cuh"
+
+namespace prc {
+
+// U, W, q and P (op_terms) of a quad's cells 2 j, 2 j + 1 from its columns.  The axis modes leave out terms that are exact
+// zeros: W is one product, whose factors s_a and v+a + v-a are returned in (W, wf) for the caller to multiply.
+template <int MODE, typename T, typename P2 = typename Pair<T>::T>
+__device__ __forceinline__ void quad_terms(const QuadCols<T>& Q, const OpCoef<T>& k, const XYCoef<T>& c, int z0, int j,
+                                           P2& U, P2& W, P2& wf, P2& q, P2& PP) {
     constexpr bool LOCAL = MODE == MG_LOCAL;
-    const V(&c)[6] = Q.c;
-    const V(&XP)[6] = Q.XP;
-    const V(&XM)[6] = Q.XM;
-    const V(&YP)[6] = Q.YP;
-    const V(&YM)[6] = Q.YM;
-    const V(&PP)[4] = Q.PP;
-    const V(&MM)[4] = Q.MM;
-    const V(&MP)[4] = Q.MP;
-    const V(&PM)[4] = Q.PM;
-    const A ih0 = (A)s.ih2[0], ih1 = (A)s.ih2[1], ih2 = (A)s.ih2[2];
-    A p0, p1, p2b;
-    if (LOCAL) {
-        p0 = (A)x + (A)s.off[0];
-        p1 = (A)y + (A)s.off[1];
-        p2b = (A)z0 + (A)s.off[2];
+    typedef Pair<T> P;
+    const int i = 2 * j;
+    const P2 p2 = P::make(z_p2<LOCAL>(k, z0 + i), z_p2<LOCAL>(k, z0 + i + 1)), s2 = P::mul(p2, p2);
+    const P2 xp = P::make(Q.XP[i + 1], Q.XP[i + 2]), xm = P::make(Q.XM[i + 1], Q.XM[i + 2]);
+    const P2 yp = P::make(Q.YP[i + 1], Q.YP[i + 2]), ym = P::make(Q.YM[i + 1], Q.YM[i + 2]);
+    const P2 zp = P::make(Q.c[i + 2], Q.c[i + 3]), zm = P::make(Q.c[i], Q.c[i + 1]);
+    if constexpr (MODE >= MG_AXIS0) {
+        const P2 Sx = P::add(xp, xm), Sy = P::add(yp, ym), Sz = P::add(zp, zm);
+        U = P::fma(both(k.ih0), Sx, P::mul(both(k.ih1), Sy));
+        U = P::fma(both(k.ih2), Sz, U);
+        W = MODE == MG_AXIS0 ? Sx : (MODE == MG_AXIS1 ? Sy : Sz);
+        wf = MODE == MG_AXIS0 ? both(c.s0) : (MODE == MG_AXIS1 ? both(c.s1) : s2);
+        q = P::fma(both(k.h22), s2, both(c.q01));
+        PP = P::add(both(c.P01), s2);
     } else {
-        p0 = (A)s.losh[0];
-        p1 = (A)s.losh[1];
-        p2b = (A)s.losh[2];
+        const P2 exy = P::sub(P::add(P::make(Q.PP[i], Q.PP[i + 1]), P::make(Q.MM[i], Q.MM[i + 1])),
+                              P::add(P::make(Q.MP[i], Q.MP[i + 1]), P::make(Q.PM[i], Q.PM[i + 1])));
+        const P2 exz = P::sub(P::add(P::make(Q.XP[i + 2], Q.XP[i + 3]), P::make(Q.XM[i], Q.XM[i + 1])),
+                              P::add(P::make(Q.XM[i + 2], Q.XM[i + 3]), P::make(Q.XP[i], Q.XP[i + 1])));
+        const P2 eyz = P::sub(P::add(P::make(Q.YP[i + 2], Q.YP[i + 3]), P::make(Q.YM[i], Q.YM[i + 1])),
+                              P::add(P::make(Q.YM[i + 2], Q.YM[i + 3]), P::make(Q.YP[i], Q.YP[i + 1])));
+        op_terms<LOCAL>(k, c, p2, s2, xp, xm, yp, ym, zp, zm, exy, exz, eyz, U, W, q, PP);
     }
-    const A s0 = p0 * p0, s1 = p1 * p1;
-    const A q01 = (A)s.h2[0] * s0 + (A)s.h2[1] * s1, P01 = s0 + s1;
-    const A e01 = (A)0.5 * p0 * p1, hp0 = (A)0.5 * p0, hp1 = (A)0.5 * p1;
+}
+
+// The damped-Jacobi values of a quad from its columns.
+template <int MODE, typename T>
+__device__ __forceinline__ void quad_jacobi(const QuadCols<T>& Q, const OpCoef<T>& k, T w, int x, int y, int z0,
+                                            const T (&f)[4], T (&o)[4]) {
+    typedef Pair<T> P;
+    const XYCoef<T> c = xy_coef<MODE == MG_LOCAL>(k, x, y);
 #pragma unroll
-    for (int k = 0; k < 4; k++) {
-        const A p2 = LOCAL ? p2b + (A)k : p2b;
-        const A s2 = p2 * p2;
-        const A xpv = (A)XP[k + 1], xmv = (A)XM[k + 1], ypv = (A)YP[k + 1], ymv = (A)YM[k + 1];
-        const A zpv = (A)c[k + 2], zmv = (A)c[k];
-        if constexpr (MODE >= MG_AXIS0) {
-            U[k] = ih0 * (xpv + xmv) + ih1 * (ypv + ymv) + ih2 * (zpv + zmv);
-            if constexpr (MODE == MG_AXIS0) W[k] = s0 * (xpv + xmv);
-            else if constexpr (MODE == MG_AXIS1) W[k] = s1 * (ypv + ymv);
-            else W[k] = s2 * (zpv + zmv);
-            qq[k] = q01 + (A)s.h2[2] * s2;
-            P[k] = P01 + s2;
-            continue;
-        }
-        const A exy = ((A)PP[k] + (A)MM[k]) - ((A)MP[k] + (A)PM[k]);
-        const A exz = ((A)XP[k + 2] + (A)XM[k]) - ((A)XM[k + 2] + (A)XP[k]);
-        const A eyz = ((A)YP[k + 2] + (A)YM[k]) - ((A)YM[k + 2] + (A)YP[k]);
-        U[k] = ih0 * (xpv + xmv) + ih1 * (ypv + ymv) + ih2 * (zpv + zmv);
-        A w;
-        if (LOCAL)
-            w = (s0 + p0) * xpv + (s0 - p0) * xmv + (s1 + p1) * ypv + (s1 - p1) * ymv + (s2 + p2) * zpv +
-                (s2 - p2) * zmv;
-        else
-            w = s0 * (xpv + xmv) + s1 * (ypv + ymv) + s2 * (zpv + zmv);
-        W[k] = w + e01 * exy + hp0 * p2 * exz + hp1 * p2 * eyz;
-        qq[k] = q01 + (A)s.h2[2] * s2;
-        P[k] = P01 + s2;
+    for (int j = 0; j < 2; j++) {
+        typename P::T U, W, wf, q, PP;
+        quad_terms<MODE>(Q, k, c, z0, j, U, W, wf, q, PP);
+        if (MODE >= MG_AXIS0) W = P::mul(wf, W);
+        const typename P::T r = op_jacobi(k, P::make(f[2 * j], f[2 * j + 1]), P::make(Q.c[2 * j + 1], Q.c[2 * j + 2]), U, W,
+                                          q, PP, w);
+        o[2 * j] = r.x, o[2 * j + 1] = r.y;
     }
 }
 
-
-template <typename A, typename V, typename S, int MODE>
-__device__ __forceinline__ void quad_terms(const V* __restrict__ v, const Stencil<S>& s, const Quad& q, A (&U)[4],
-                                           A (&W)[4], A (&qq)[4], A (&P)[4]) {
-    QuadCols<V> Q;
-    quad_load<MODE>(v, s, q, Q);
-    quad_compute<A, V, S, MODE>(Q, s, q.x, q.y, q.z0, U, W, qq, P);
-}
-
-template <typename T> __device__ __forceinline__ T quotient(T a, T b) {
-    if constexpr (sizeof(T) == 4) return __fdividef(a, b);   // FP32 sweeps: fast reciprocal (2 ulp)
-    else return a / b;
-}
-
-// quad_compute's terms where v is identically zero (the first sweep of a V-cycle started from zero).
-template <typename T, bool LOCAL>
-__device__ __forceinline__ void quad_zero_terms(const Stencil<T>& s, int x, int y, int z0, T (&U)[4], T (&W)[4],
-                                                T (&qq)[4], T (&P)[4], T (&vc)[4]) {
-    const T p0 = LOCAL ? (T)x + s.off[0] : s.losh[0], p1 = LOCAL ? (T)y + s.off[1] : s.losh[1];
+// The same where v is identically zero (the first sweep of a V-cycle started from zero): w q f / den, with q and P
+// summed in their own order (local: h_0^2 p_0^2 and h_1^2 p_1^2 as (h^2 p) p).
+template <bool LOCAL, typename T>
+__device__ __forceinline__ void quad_zero(const OpCoef<T>& k, T w, int x, int y, int z0, const T (&f)[4], T (&o)[4]) {
+    typedef Pair<T> P;
+    typedef typename P::T P2;
+    XYCoef<T> c = xy_coef<LOCAL>(k, x, y);
+    if (LOCAL) {
+        const T p0 = rn_add((T)x, k.off0), p1 = rn_add((T)y, k.off1);
+        c.q01 = fma_rn(rn_mul(k.h21, p1), p1, rn_mul(rn_mul(k.h20, p0), p0));
+        c.P01 = fma_rn(p1, p1, c.s0);
+    }
+    const P2 zero = both((T)0);
 #pragma unroll
-    for (int k = 0; k < 4; k++) {
-        const T p2 = LOCAL ? (T)(z0 + k) + s.off[2] : s.losh[2];
-        const T s2 = p2 * p2;
-        qq[k] = s.h2[0] * p0 * p0 + s.h2[1] * p1 * p1 + s.h2[2] * s2;
-        P[k] = p0 * p0 + p1 * p1 + s2;
-        U[k] = W[k] = vc[k] = (T)0;
+    for (int j = 0; j < 2; j++) {
+        const P2 p2 = LOCAL ? P::make(rn_add((T)(z0 + 2 * j), k.off2), rn_add((T)(z0 + 2 * j + 1), k.off2)) : both(k.off2);
+        const P2 s2 = P::mul(p2, p2), q = P::fma(both(k.h22), s2, both(c.q01)), PP = P::add(both(c.P01), s2);
+        const P2 r = op_jacobi(k, P::make(f[2 * j], f[2 * j + 1]), zero, zero, zero, q, PP, w);
+        o[2 * j] = r.x, o[2 * j + 1] = r.y;
     }
 }
 
-// The damped-Jacobi update of a quad: jac = (q (f + U) + beta W) / (2 (q sum 1/h^2 + beta P)),
-// o = v + w (jac - v).
-template <typename T>
-__device__ __forceinline__ void quad_blend(const Stencil<T>& s, T w, const T (&fv)[4], const T (&vc)[4],
-                                           const T (&U)[4], const T (&W)[4], const T (&qq)[4], const T (&P)[4],
-                                           T (&o)[4]) {
-    const T sih = s.ih2[0] + s.ih2[1] + s.ih2[2];
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-        const T jac = quotient<T>(qq[k] * (fv[k] + U[k]) + s.beta * W[k], (T)2 * (qq[k] * sih + s.beta * P[k]));
-        o[k] = vc[k] + w * (jac - vc[k]);
+template <typename T> __device__ __forceinline__ void store4(T* p, const T (&o)[4]) {
+    if constexpr (sizeof(T) == 4) {
+        *(float4*)p = make_float4(o[0], o[1], o[2], o[3]);
+    } else {
+        ((double2*)p)[0] = make_double2(o[0], o[1]);
+        ((double2*)p)[1] = make_double2(o[2], o[3]);
     }
 }
 
-// Damped-Jacobi sweep of four cells per thread:
-//   jac = (f + S) / (2 sum G) = (q (f + U) + beta W) / (2 (q sum 1/h^2 + beta P)),
-//   vout = v + w (jac - v).
+// Damped-Jacobi sweep of four cells per thread: the axis modes, rows too long for march_kernel, and (zero_v)
+// every sweep from an identically zero v.
+// acc (optional): the sweep's result is added to it instead of being stored (OP_JACOBI_ADD).
 template <typename T, int MODE>
 __global__ void __launch_bounds__(256) jacobi_sweep4(const T* __restrict__ v, const T* __restrict__ f,
-                                                     T* __restrict__ vout, Stencil<T> s, T w, int zero_v) {
+                                                     T* __restrict__ vout, double* __restrict__ acc, Stencil<T> s, T w,
+                                                     int zero_v) {
     pdl_trigger();
     pdl_wait();
     Quad q;
     if (!quad_of(s.n, q)) return;
     const int64_t bo = batch_offset(s.n);
     v += bo, f += bo, vout += bo;
-    T fv[4], vc[4], U[4], W[4], qq[4], P[4];
+    const OpCoef<T> k = op_coef<MODE == MG_LOCAL>(s);
+    T fv[4], o[4];
     load4(f + q.c + q.z0, fv);
     if (zero_v) {
-        quad_zero_terms<T, MODE == MG_LOCAL>(s, q.x, q.y, q.z0, U, W, qq, P, vc);
+        quad_zero<MODE == MG_LOCAL>(k, w, q.x, q.y, q.z0, fv, o);
     } else {
-        quad_terms<T, T, T, MODE>(v, s, q, U, W, qq, P);
-        load4(v + q.c + q.z0, vc);
+        QuadCols<T> Q;
+        quad_load<MODE>(v, s, q, Q);
+        quad_jacobi<MODE>(Q, k, w, q.x, q.y, q.z0, fv, o);
     }
-    T o[4];
-    quad_blend(s, w, fv, vc, U, W, qq, P, o);
-    if constexpr (sizeof(T) == 4) {
-        *(float4*)(vout + q.c + q.z0) = make_float4(o[0], o[1], o[2], o[3]);
+    if (acc != nullptr) {
+        double* a = acc + bo + q.c + q.z0;
+        double t[4];
+#pragma unroll
+        for (int j = 0; j < 4; j += 2) {
+            const double2 d = *(const double2*)(a + j);
+            t[j] = d.x + (double)o[j], t[j + 1] = d.y + (double)o[j + 1];
+        }
+        store4(a, t);
     } else {
-        ((double2*)(vout + q.c + q.z0))[0] = make_double2(o[0], o[1]);
-        ((double2*)(vout + q.c + q.z0))[1] = make_double2(o[2], o[3]);
+        store4(vout + q.c + q.z0, o);
     }
 }
 
@@ -466,6 +444,7 @@ __global__ void __launch_bounds__(TQ * TY, (sizeof(T) == 4 ? 6 : 4)) jacobi_swee
     const int y0 = blockIdx.y * TY, z0 = blockIdx.x * (4 * TQ);
     const int tid = threadIdx.x;
     const int64_t sx = (int64_t)n1 * n2;
+    const OpCoef<T> kc = op_coef<LOCAL>(s);
 
     // stage plane x (periodic) of v into ring slot x mod 3
     auto stage = [&](int x) {
@@ -497,17 +476,15 @@ __global__ void __launch_bounds__(TQ * TY, (sizeof(T) == 4 ? 6 : 4)) jacobi_swee
             for (int q = tid; q < SH::R1 * SH::Q1; q += SH::THREADS) {
                 const int r = q / SH::Q1, k = q % SH::Q1;
                 const int gy = wrap_mod(y0 - 1 + r, n1), gz = wrap_mod(z0 - 4 + 4 * k, n2);
-                T fv[4], vc[4], U[4], W[4], qq[4], P[4], o[4];
+                T fv[4], o[4];
                 load4(f + (int64_t)gx * sx + (int64_t)gy * n2 + gz, fv);
                 if (zero_v) {
-                    quad_zero_terms<T, LOCAL>(s, gx, gy, gz, U, W, qq, P, vc);
+                    quad_zero<LOCAL>(kc, w, gx, gy, gz, fv, o);
                 } else {
                     QuadCols<T> Q;
                     smem_cols<T, ZP>(lo, mid, hi, r + 1, 4 * k + 4, Q);
-                    quad_compute<T, T, T, LOCAL>(Q, s, gx, gy, gz, U, W, qq, P);
-                    smem_quad4(mid + (r + 1) * ZP, 4 * k + 4, vc);
+                    quad_jacobi<LOCAL ? MG_LOCAL : MG_GLOBAL>(Q, kc, w, gx, gy, gz, fv, o);
                 }
-                quad_blend(s, w, fv, vc, U, W, qq, P, o);
                 smem_store4(out + r * ZP, 4 * k + 4, o);
             }
         }
@@ -522,13 +499,11 @@ __global__ void __launch_bounds__(TQ * TY, (sizeof(T) == 4 ? 6 : 4)) jacobi_swee
             const int gy = y0 + r, gz = z0 + 4 * k;
             if (gy < n1 && gz < n2) {
                 const int64_t at = (int64_t)xo * sx + (int64_t)gy * n2 + gz;
-                T fv[4], vc[4], U[4], W[4], qq[4], P[4], o[4];
+                T fv[4], o[4];
                 load4(f + at, fv);
                 QuadCols<T> Q;
                 smem_cols<T, ZP>(lo, mid, hi, r + 1, 4 * k + 8, Q);
-                quad_compute<T, T, T, LOCAL>(Q, s, xo, gy, gz, U, W, qq, P);
-                smem_quad4(mid + (r + 1) * ZP, 4 * k + 8, vc);
-                quad_blend(s, w, fv, vc, U, W, qq, P, o);
+                quad_jacobi<LOCAL ? MG_LOCAL : MG_GLOBAL>(Q, kc, w, xo, gy, gz, fv, o);
                 if constexpr (sizeof(T) == 4) {
                     *(float4*)(vout + at) = make_float4(o[0], o[1], o[2], o[3]);
                 } else {
@@ -540,29 +515,40 @@ __global__ void __launch_bounds__(TQ * TY, (sizeof(T) == 4 ? 6 : 4)) jacobi_swee
     }
 }
 
-// r = f - A v = (f + U - 2 v sum 1/h^2) + g (W - 2 P v), g = beta / q, evaluated in type A.
-template <typename A, typename V, typename FT, typename R, typename S, int MODE>
-__global__ void __launch_bounds__(256) residual_kernel4(const V* __restrict__ v, const FT* __restrict__ f,
-                                                        R* __restrict__ r, Stencil<S> s) {
+// r = f - A v of four cells per thread, evaluated in type A and stored as R: the axis modes, and rows too long for
+// march_kernel.
+template <typename A, typename R, int MODE>
+__global__ void __launch_bounds__(256) residual_kernel4(const A* __restrict__ v, const A* __restrict__ f,
+                                                        R* __restrict__ r, Stencil<A> s) {
     pdl_trigger();
     pdl_wait();
     Quad q;
     if (!quad_of(s.n, q)) return;
     const int64_t bo = batch_offset(s.n);
     v += bo, f += bo, r += bo;
-    A U[4], W[4], qq[4], P[4];
-    quad_terms<A, V, S, MODE>(v, s, q, U, W, qq, P);
-    V vc[4];
-    FT fv[4];
-    load4(v + q.c + q.z0, vc);
+    typedef Pair<A> P;
+    QuadCols<A> Q;
+    A fv[4];
+    R o[4];
+    quad_load<MODE>(v, s, q, Q);
     load4(f + q.c + q.z0, fv);
-    const A sih2 = (A)2 * ((A)s.ih2[0] + (A)s.ih2[1] + (A)s.ih2[2]);
+    const OpCoef<A> k = op_coef<MODE == MG_LOCAL>(s);
+    const XYCoef<A> c = xy_coef<MODE == MG_LOCAL>(k, q.x, q.y);
 #pragma unroll
-    for (int k = 0; k < 4; k++) {
-        const A g = quotient<A>((A)s.beta, qq[k]);
-        const A x = (A)vc[k];
-        r[q.c + q.z0 + k] = (R)(((A)fv[k] + U[k] - sih2 * x) + g * (W[k] - (A)2 * P[k] * x));
+    for (int j = 0; j < 2; j++) {
+        typename P::T U, W, wf, qq, PP;
+        quad_terms<MODE>(Q, k, c, q.z0, j, U, W, wf, qq, PP);
+        const typename P::T v2 = P::make(Q.c[2 * j + 1], Q.c[2 * j + 2]), f2 = P::make(fv[2 * j], fv[2 * j + 1]);
+        typename P::T t;
+        if constexpr (MODE >= MG_AXIS0 && sizeof(A) == 4) {
+            t = op_residual_from(k, f2, v2, U, P::fma(wf, W, P::mul(P::mul(both((A)-2), PP), v2)), qq);
+        } else {
+            if (MODE >= MG_AXIS0) W = P::mul(wf, W);
+            t = op_residual(k, f2, v2, U, W, qq, PP);
+        }
+        o[2 * j] = (R)t.x, o[2 * j + 1] = (R)t.y;
     }
+    store4(r + q.c + q.z0, o);
 }
 
 // r = f - A v, evaluated in type A (double for the mixed-precision defect), stored as R.
@@ -593,14 +579,13 @@ template <typename T> static decltype(&jacobi_sweep4<T, MG_GLOBAL>) sweep4_kerne
     default: return jacobi_sweep4<T, MG_GLOBAL>;
     }
 }
-template <typename A, typename V, typename FT, typename R, typename S>
-static decltype(&residual_kernel4<A, V, FT, R, S, MG_GLOBAL>) residual4_kernel(int mode) {
+template <typename A, typename R> static decltype(&residual_kernel4<A, R, MG_GLOBAL>) residual4_kernel(int mode) {
     switch (mode) {
-    case MG_LOCAL: return residual_kernel4<A, V, FT, R, S, MG_LOCAL>;
-    case MG_AXIS0: return residual_kernel4<A, V, FT, R, S, MG_AXIS0>;
-    case MG_AXIS1: return residual_kernel4<A, V, FT, R, S, MG_AXIS1>;
-    case MG_AXIS2: return residual_kernel4<A, V, FT, R, S, MG_AXIS2>;
-    default: return residual_kernel4<A, V, FT, R, S, MG_GLOBAL>;
+    case MG_LOCAL: return residual_kernel4<A, R, MG_LOCAL>;
+    case MG_AXIS0: return residual_kernel4<A, R, MG_AXIS0>;
+    case MG_AXIS1: return residual_kernel4<A, R, MG_AXIS1>;
+    case MG_AXIS2: return residual_kernel4<A, R, MG_AXIS2>;
+    default: return residual_kernel4<A, R, MG_GLOBAL>;
     }
 }
 
@@ -675,6 +660,112 @@ __global__ void __launch_bounds__(256) prolong_kernel(const TI* __restrict__ coa
     }
 }
 
+// ---- restriction and prolongation, two coarse cells along z per thread (fine n2 % 4 == 0, aligned meshes) ----
+// Bound by memory: a fine mesh is read (and written) in 16-byte vectors, four fine cells a row instead of one.
+template <typename T> __device__ __forceinline__ void load2(const T* __restrict__ p, T (&o)[2]) {
+    if constexpr (sizeof(T) == 4) {
+        const float2 q = __ldg((const float2*)p);
+        o[0] = q.x, o[1] = q.y;
+    } else {
+        const double2 q = __ldg((const double2*)p);
+        o[0] = q.x, o[1] = q.y;
+    }
+}
+
+// Launch over (n0, n1, n2 / 2) of the coarse shape; nc: the coarse shape.
+__device__ __forceinline__ bool coarse_pair(const int nc[3], int& x, int& y, int& z) {
+    z = 2 * (blockIdx.x * blockDim.x + threadIdx.x);
+    y = blockIdx.y * blockDim.y + threadIdx.y;
+    x = gridDim.z == (unsigned)nc[0] ? (int)blockIdx.z : (int)(blockIdx.z % nc[0]);
+    return z < nc[2] && y < nc[1];
+}
+
+// The order of the sum is reduce_kernel's (its weights are powers of two: every product is exact).
+template <typename T>
+__global__ void __launch_bounds__(256) reduce_pair(const T* __restrict__ fine, T* __restrict__ coarse, Dims nf) {
+    pdl_trigger();
+    pdl_wait();
+    const int nc[3] = {nf.n[0] / 2, nf.n[1] / 2, nf.n[2] / 2};
+    int x, y, z;
+    if (!coarse_pair(nc, x, y, z)) return;
+    const int64_t bc = batch_offset(nc);
+    fine += 8 * bc, coarse += bc;
+    const int X[3] = {wrap_dn(2 * x, nf.n[0]), 2 * x, wrap_up(2 * x, nf.n[0])};
+    const int Y[3] = {wrap_dn(2 * y, nf.n[1]), 2 * y, wrap_up(2 * y, nf.n[1])};
+    const int zm = z == 0 ? nf.n[2] - 1 : 2 * z - 1;
+    T acc[2] = {0, 0};
+#pragma unroll
+    for (int a = 0; a < 3; a++)
+#pragma unroll
+        for (int b = 0; b < 3; b++) {
+            const T* row = fine + ((int64_t)X[a] * nf.n[1] + Y[b]) * nf.n[2];
+            T m[4];
+            load4(row + 2 * z, m);
+            const T left = __ldg(row + zm);
+            const int side = (a != 1) + (b != 1);
+            const T wc = (T)(8 >> side), we = (T)(4 >> side);
+            acc[0] = fma_rn(we, m[1], fma_rn(wc, m[0], fma_rn(we, left, acc[0])));
+            acc[1] = fma_rn(we, m[3], fma_rn(wc, m[2], fma_rn(we, m[1], acc[1])));
+        }
+    T* o = coarse + ((int64_t)x * nc[1] + y) * nc[2] + z;
+    if constexpr (sizeof(T) == 4) *(float2*)o = make_float2(acc[0] / 64, acc[1] / 64);
+    else *(double2*)o = make_double2(acc[0] / 64, acc[1] / 64);
+}
+
+// ADD: fine += the prolonged coarse mesh, else fine = it.
+template <typename T, bool ADD>
+__global__ void __launch_bounds__(256) prolong_pair(const T* __restrict__ coarse, T* __restrict__ fine, Dims nc) {
+    pdl_trigger();
+    pdl_wait();
+    int x, y, z;
+    if (!coarse_pair(nc.n, x, y, z)) return;
+    const int64_t bc = batch_offset(nc.n);
+    coarse += bc, fine += 8 * bc;
+    const int64_t nf1 = 2 * nc.n[1], nf2 = 2 * nc.n[2];
+    const int xs[2] = {x, wrap_up(x, nc.n[0])}, ys[2] = {y, wrap_up(y, nc.n[1])}, zn = z + 2 == nc.n[2] ? 0 : z + 2;
+    T c[2][2][3];
+#pragma unroll
+    for (int a = 0; a < 2; a++)
+#pragma unroll
+        for (int b = 0; b < 2; b++) {
+            const T* row = coarse + ((int64_t)xs[a] * nc.n[1] + ys[b]) * nc.n[2];
+            T t[2];
+            load2(row + z, t);
+            c[a][b][0] = t[0], c[a][b][1] = t[1], c[a][b][2] = __ldg(row + zn);
+        }
+#pragma unroll
+    for (int ex = 0; ex < 2; ex++)
+#pragma unroll
+        for (int ey = 0; ey < 2; ey++) {
+            T* dst = fine + ((2 * x + ex) * nf1 + (2 * y + ey)) * nf2 + 2 * z;
+            T o[4];
+            if constexpr (ADD) {
+                if constexpr (sizeof(T) == 4) {
+                    const float4 q = *(const float4*)dst;
+                    o[0] = q.x, o[1] = q.y, o[2] = q.z, o[3] = q.w;
+                } else {
+                    const double2 q = *(const double2*)dst, w = *((const double2*)dst + 1);
+                    o[0] = q.x, o[1] = q.y, o[2] = w.x, o[3] = w.y;
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                // the mean of the corners, summed in prolong_kernel's order
+                const int d = j / 2, ez = j & 1;
+                T t = 0;
+#pragma unroll
+                for (int a = 0; a <= ex; a++)
+#pragma unroll
+                    for (int b = 0; b <= ey; b++)
+#pragma unroll
+                        for (int e = 0; e <= ez; e++) t = rn_add(t, c[a][b][d + e]);
+                t = rn_mul(t, (T)1 / (T)((1 + ex) * (1 + ey) * (1 + ez)));
+                o[j] = ADD ? rn_add(o[j], t) : t;
+            }
+            store4(dst, o);
+        }
+}
+
 template <typename TI, typename TO>
 __global__ void convert_kernel(const TI* __restrict__ in, TO* __restrict__ out, int64_t n) {
     pdl_trigger();
@@ -722,6 +813,59 @@ static Grid3 grid3_quad(const int n[3], int count = 1) {
 }
 static bool quad_ok(const int n[3], const void* a, const void* b, const void* c) {
     return n[2] % 4 == 0 && (((uintptr_t)a | (uintptr_t)b | (uintptr_t)c) & 15) == 0;
+}
+
+// March kernels: usable for the 19-point operator (local or oblique line of sight) where the quad kernels are
+// and a row holds a tile.
+// Below MARCH_MIN_BYTES of v the quad kernels are as fast (64^3 FP32, 1 MB: 3.2 against 3.7 us, the march's pipeline
+// fill; 96^3 FP32, 3.5 MB: 6.0 against 4.7 us; 64^3 FP64, 2 MB: 4.2 against 4.0 us).
+constexpr int64_t MARCH_MIN_BYTES = 3 << 19;
+template <typename A> static bool march_ok(const Stencil<A>& s, int count) {
+    return mg_mode(s) <= MG_LOCAL && s.n[2] >= 4 * MarchVZ<A>::value && (int64_t)s.n[0] * count <= 65535 &&
+           (int64_t)s.n[0] * s.n[1] * s.n[2] * count * (int64_t)sizeof(A) >= MARCH_MIN_BYTES;
+}
+
+template <typename A, typename OT, int OP>
+static cudaError_t launch_march(const A* v, const A* f, OT* out, double* acc, const Stencil<A>& s, A w, int count,
+                                cudaStream_t st) {
+    const MarchSplit sp = march_split<A>(s.n, count);
+    void (*kernel)(const A*, const A*, OT*, double*, Stencil<A>, A, MarchSplit) = nullptr;
+    size_t smem = 0;
+#define MARCH_CASE(LZ)                                                                                  \
+    case LZ:                                                                                            \
+        kernel = s.local ? march_kernel<A, OT, LZ, true, OP> : march_kernel<A, OT, LZ, false, OP>;      \
+        smem = (size_t)MARCH_STAGES * MarchTile<A, LZ>::STAGE;                                          \
+        break;
+    switch (sp.lz) {
+        MARCH_CASE(32)
+        MARCH_CASE(16)
+        MARCH_CASE(8)
+        MARCH_CASE(4)
+        default: return cudaErrorInvalidValue;
+    }
+#undef MARCH_CASE
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    return launch_pdl(kernel, dim3(sp.zsegs, sp.ytiles, sp.nslab * count), dim3(MARCH_THREADS), smem, st, v, f, out, acc,
+                      s, w, sp);
+}
+
+// Coarse (nf / 2) from fine, and fine (2 nc) from coarse, over `count` meshes.
+template <typename T>
+static cudaError_t launch_reduce(const T* fine, T* coarse, const int nf[3], int count, cudaStream_t st) {
+    const Dims d = {{nf[0], nf[1], nf[2]}};
+    const int half[3] = {nf[0] / 2, nf[1] / 2, nf[2] / 4};
+    const bool pair = nf[2] % 4 == 0 && (((uintptr_t)fine | (uintptr_t)coarse) & 15) == 0;
+    const Grid3 g = pair ? grid3(half, count) : grid3_coarse(nf, count);
+    return launch_pdl(pair ? reduce_pair<T> : reduce_kernel<T, T, T>, g.grid, g.block, 0, st, fine, coarse, d);
+}
+template <typename T, bool ADD>
+static cudaError_t launch_prolong(const T* coarse, T* fine, const int nc[3], int count, cudaStream_t st) {
+    const Dims d = {{nc[0], nc[1], nc[2]}};
+    const int half[3] = {nc[0], nc[1], nc[2] / 2};
+    const bool pair = nc[2] % 2 == 0 && (((uintptr_t)fine | (uintptr_t)coarse) & 15) == 0;
+    const Grid3 g = grid3(pair ? half : nc, count);
+    return launch_pdl(pair ? prolong_pair<T, ADD> : prolong_kernel<T, T, T, ADD>, g.grid, g.block, 0, st, coarse, fine, d);
 }
 
 // Tile of the temporal-blocked sweeps: TB_TY rows x 4 TB_TQ cells.
@@ -954,7 +1098,8 @@ template <typename T> struct MGRunner {
     // other buffer (the pointers are swapped instead of copying back).  zero_first: v known zero.
     // Pairs of sweeps run as one temporal-blocked pass when the tuning table's "mg_jacobi" (FP32) or
     // "mg_jacobi_f64" entry for the level (keyed by n0) is a slab length > 0 (mg_tb_default otherwise).
-    int jacobi(int l, T*& v, const T* f, T*& tmp, int niter, bool zero_first) {
+    // acc (optional): the last sweep adds its result to acc, and nothing is left in v.
+    int jacobi(int l, T*& v, const T* f, T*& tmp, int niter, bool zero_first, double* acc = nullptr) {
         Stencil<T> s = stencil(l);
         const int64_t N = L[l].size() * count;
         const Grid3 g = grid3(L[l].n, count);
@@ -969,7 +1114,7 @@ template <typename T> struct MGRunner {
             const int nslab = (L[l].n[0] + slab - 1) / slab;
             const dim3 grid((L[l].n[2] + 4 * TB_TQ - 1) / (4 * TB_TQ), (L[l].n[1] + TB_TY - 1) / TB_TY, nslab * count);
             if ((int64_t)nslab * count <= 65535) {
-                for (; it + 1 < niter; it += 2) {
+                for (; it + 1 < (acc != nullptr ? niter - 1 : niter); it += 2) {
                     const bool z0 = zero_first && it == 0;
                     PRC_LAUNCH_B("mg_jacobi2", st, (double)N * sizeof(T) * (z0 ? 2 : 3),
                                  launch_pdl((s.local ? jacobi_sweep2_tb<T, true, TB_TY, TB_TQ>
@@ -980,12 +1125,25 @@ template <typename T> struct MGRunner {
         }
         for (; it < niter; it++) {
             const bool z0 = zero_first && it == 0;
-            if (quad)
-                PRC_LAUNCH_B("mg_jacobi", st, (double)N * sizeof(T) * (z0 ? 2 : 3),
-                             launch_pdl(sweep4_kernel<T>(mg_mode(s)), gq.grid, gq.block, 0, st, v, f, tmp, s, (T)P.damping, z0));
-            else
+            double* a = it + 1 == niter ? acc : nullptr;
+            const double bytes = (double)N * (sizeof(T) * (z0 ? 1 : 2) + (a != nullptr ? 16 : sizeof(T)));
+            if (quad && !z0 && march_ok(s, count)) {
+                if (a != nullptr)
+                    PRC_LAUNCH_B("mg_jacobi_add", st, bytes,
+                                 (launch_march<T, T, OP_JACOBI_ADD>(v, f, tmp, a, s, (T)P.damping, count, st)));
+                else
+                    PRC_LAUNCH_B("mg_jacobi", st, bytes,
+                                 (launch_march<T, T, OP_JACOBI>(v, f, tmp, nullptr, s, (T)P.damping, count, st)));
+            } else if (quad) {
+                PRC_LAUNCH_B(a != nullptr ? "mg_jacobi_add" : "mg_jacobi", st, bytes,
+                             launch_pdl(sweep4_kernel<T>(mg_mode(s)), gq.grid, gq.block, 0, st, v, f, tmp, a, s, (T)P.damping, z0));
+            } else {
                 PRC_LAUNCH_B("mg_jacobi", st, (double)N * sizeof(T) * (z0 ? 2 : 3),
                              launch_pdl(jacobi_sweep<T, T>, g.grid, g.block, 0, st, v, f, tmp, s, (T)P.damping, z0));
+                if (a != nullptr)
+                    PRC_LAUNCH_B("mg_correct_fp64", st, (16.0 + sizeof(T)) * N,
+                                 launch_pdl(add_kernel<double, T>, grid_for(N), 256, 0, st, a, tmp, N));
+            }
             std::swap(v, tmp);
         }
         PRC_CHECK_LAUNCH();
@@ -1023,34 +1181,49 @@ template <typename T> struct MGRunner {
     }
 
     // Recursive V-cycle on level l: v (B[l].v, or the caller's level-0 pointer) with right-hand side f.
-    int vcycle(int l, T*& v, const T* f, bool v_zero) {
+    // acc (optional): the cycle's result is added to it; where the last step could do so itself, v holds nothing.
+    int vcycle(int l, T*& v, const T* f, bool v_zero, double* acc = nullptr) {
         bool small = false;
         PRC_TRY(small_vcycle(l, v, f, v_zero, &small));
-        if (small) return PRC_OK;
+        if (small || P.jn == 0) {
+            if (!small) PRC_TRY(vcycle_steps(l, v, f, v_zero, nullptr));
+            if (acc != nullptr) {
+                const int64_t N = L[l].size() * count;
+                PRC_LAUNCH_B("mg_correct_fp64", st, 20.0 * N,
+                             launch_pdl(add_kernel<double, T>, grid_for(N), 256, 0, st, acc, v, N));
+                PRC_CHECK_LAUNCH();
+            }
+            return PRC_OK;
+        }
+        return vcycle_steps(l, v, f, v_zero, acc);
+    }
+
+    int vcycle_steps(int l, T*& v, const T* f, bool v_zero, double* acc) {
         PRC_TRY(jacobi(l, v, f, B[l].tmp, P.jn, v_zero));
         if (l + 1 < (int)L.size()) {
             Stencil<T> s = stencil(l);
             const int64_t N = L[l].size() * count;
-            const Grid3 g = grid3(L[l].n, count), gc = grid3_coarse(L[l].n, count);
-            if (quad_ok(L[l].n, v, f, B[l].r)) {
+            const Grid3 g = grid3(L[l].n, count);
+            if (quad_ok(L[l].n, v, f, B[l].r) && march_ok(s, count)) {
+                PRC_LAUNCH_B("mg_residual", st, 3.0 * N * sizeof(T),
+                             (launch_march<T, T, OP_RESIDUAL>(v, f, B[l].r, nullptr, s, (T)0, count, st)));
+            } else if (quad_ok(L[l].n, v, f, B[l].r)) {
                 const Grid3 gq = grid3_quad(L[l].n, count);
                 PRC_LAUNCH_B("mg_residual", st, 3.0 * N * sizeof(T),
-                             launch_pdl(residual4_kernel<T, T, T, T, T>(mg_mode(s)), gq.grid, gq.block, 0, st, v, f, B[l].r, s));
+                             launch_pdl(residual4_kernel<T, T>(mg_mode(s)), gq.grid, gq.block, 0, st, v, f, B[l].r, s));
             } else {
                 PRC_LAUNCH_B("mg_residual", st, 3.0 * N * sizeof(T),
                              launch_pdl(residual_kernel<T, T, T, T, T>, g.grid, g.block, 0, st, v, f, B[l].r, s));
             }
-            Dims nf = {{L[l].n[0], L[l].n[1], L[l].n[2]}};
             PRC_LAUNCH_B("mg_reduce", st, (double)(N + L[l + 1].size() * count) * sizeof(T),
-                         launch_pdl(reduce_kernel<T, T, T>, gc.grid, gc.block, 0, st, B[l].r, B[l + 1].f, nf));
+                         launch_reduce(B[l].r, B[l + 1].f, L[l].n, count, st));
             PRC_CHECK_LAUNCH();
             PRC_TRY(vcycle(l + 1, B[l + 1].v, B[l + 1].f, true));
-            Dims nc = {{L[l + 1].n[0], L[l + 1].n[1], L[l + 1].n[2]}};
             PRC_LAUNCH_B("mg_prolong_add", st, (double)(2 * N + L[l + 1].size() * count) * sizeof(T),
-                         launch_pdl(prolong_kernel<T, T, T, true>, gc.grid, gc.block, 0, st, B[l + 1].v, v, nc));
+                         (launch_prolong<T, true>(B[l + 1].v, v, L[l + 1].n, count, st)));
             PRC_CHECK_LAUNCH();
         }
-        return jacobi(l, v, f, B[l].tmp, P.jn, false);
+        return jacobi(l, v, f, B[l].tmp, P.jn, false, acc);
     }
 };
 
@@ -1062,10 +1235,8 @@ template <typename T> static int fmg_plain(MGRunner<T>& R, const T* f0, T* v0) {
     R.B[0].f = const_cast<T*>(f0);
     const int cnt = R.count;
     for (int l = 0; l + 1 < nl; l++) {
-        Dims nf = {{R.L[l].n[0], R.L[l].n[1], R.L[l].n[2]}};
-        const Grid3 gc = grid3_coarse(R.L[l].n, cnt);
         PRC_LAUNCH_B("mg_reduce", st, (double)(R.L[l].size() + R.L[l + 1].size()) * cnt * sizeof(T),
-                     launch_pdl(reduce_kernel<T, T, T>, gc.grid, gc.block, 0, st, R.B[l].f, R.B[l + 1].f, nf));
+                     launch_reduce(R.B[l].f, R.B[l + 1].f, R.L[l].n, cnt, st));
     }
     PRC_CHECK_LAUNCH();
     // the FMG solution of level l >= 1 lives in B[l].v; level 0 starts in v0 and may end in
@@ -1076,10 +1247,8 @@ template <typename T> static int fmg_plain(MGRunner<T>& R, const T* f0, T* v0) {
         if (l == nl - 1) {
             if (cudaMemsetAsync(v, 0, R.L[l].size() * cnt * sizeof(T), st) != cudaSuccess) return PRC_ERR_CUDA;
         } else {
-            Dims nc = {{R.L[l + 1].n[0], R.L[l + 1].n[1], R.L[l + 1].n[2]}};
-            const Grid3 gc = grid3(R.L[l + 1].n, cnt);
             PRC_LAUNCH_B("mg_prolong", st, (double)(R.L[l].size() + R.L[l + 1].size()) * cnt * sizeof(T),
-                         launch_pdl(prolong_kernel<T, T, T, false>, gc.grid, gc.block, 0, st, R.B[l + 1].v, v, nc));
+                         (launch_prolong<T, false>(R.B[l + 1].v, v, R.L[l + 1].n, cnt, st)));
             PRC_CHECK_LAUNCH();
         }
         for (int it = 0; it < R.P.vn; it++) PRC_TRY(R.vcycle(l, v, R.B[l].f, l == nl - 1 && it == 0));
@@ -1203,10 +1372,8 @@ int solve_mixed(const int32_t nmesh[3], const Params& P, void* ws, cudaStream_t 
     R.st = st;
     R.count = count;
     for (int l = 0; l + 1 < nl; l++) {
-        Dims nf = {{m.L[l].n[0], m.L[l].n[1], m.L[l].n[2]}};
-        const Grid3 gc = grid3_coarse(m.L[l].n, count);
         PRC_LAUNCH_B("mg_reduce", st, 8.0 * (m.L[l].size() + m.L[l + 1].size()) * count,
-                     launch_pdl(reduce_kernel<double, double, double>, gc.grid, gc.block, 0, st, m.f64[l], m.f64[l + 1], nf));
+                     launch_reduce(m.f64[l], m.f64[l + 1], m.L[l].n, count, st));
     }
     PRC_CHECK_LAUNCH();
     for (int l = nl - 1; l >= 0; l--) {
@@ -1215,29 +1382,27 @@ int solve_mixed(const int32_t nmesh[3], const Params& P, void* ws, cudaStream_t 
         if (l == nl - 1) {
             if (cudaMemsetAsync(m.v64[l], 0, N * 8, st) != cudaSuccess) return PRC_ERR_CUDA;
         } else {
-            Dims nc = {{m.L[l + 1].n[0], m.L[l + 1].n[1], m.L[l + 1].n[2]}};
-            const Grid3 gc = grid3(m.L[l + 1].n, count);
             PRC_LAUNCH_B("mg_prolong", st, 8.0 * (m.L[l].size() + m.L[l + 1].size()) * count,
-                         launch_pdl(prolong_kernel<double, double, double, false>, gc.grid, gc.block, 0, st, m.v64[l + 1],
-                                                                                                  m.v64[l], nc));
+                         (launch_prolong<double, false>(m.v64[l + 1], m.v64[l], m.L[l + 1].n, count, st)));
         }
         Stencil<double> s64 = make_stencil<double>(m.L[l].n, P.boxsize, P.boxcenter, P.beta,
                                                    P.has_los ? P.los : nullptr);
         for (int it = 0; it < P.vn; it++) {
             // defect in FP64 (stored FP32 as the inner V-cycle's right-hand side)
-            if (quad_ok(m.L[l].n, m.v64[l], m.f64[l], R.B[l].f)) {
+            if (quad_ok(m.L[l].n, m.v64[l], m.f64[l], R.B[l].f) && march_ok(s64, count)) {
+                PRC_LAUNCH_B("mg_residual_fp64", st, 20.0 * N,
+                             (launch_march<double, float, OP_RESIDUAL>(m.v64[l], m.f64[l], R.B[l].f, nullptr,
+                                                                               s64, 0., count, st)));
+            } else if (quad_ok(m.L[l].n, m.v64[l], m.f64[l], R.B[l].f)) {
                 const Grid3 gq = grid3_quad(m.L[l].n, count);
                 PRC_LAUNCH_B("mg_residual_fp64", st, 20.0 * N,
-                             launch_pdl(residual4_kernel<double, double, double, float, double>(mg_mode(s64)), gq.grid, gq.block, 0, st, m.v64[l], m.f64[l], R.B[l].f, s64));
+                             launch_pdl(residual4_kernel<double, float>(mg_mode(s64)), gq.grid, gq.block, 0, st, m.v64[l], m.f64[l], R.B[l].f, s64));
             } else {
                 PRC_LAUNCH_B("mg_residual_fp64", st, 20.0 * N,
                              launch_pdl(residual_kernel<double, double, double, float, double>, g.grid, g.block, 0, st, m.v64[l], m.f64[l], R.B[l].f, s64));
             }
             PRC_CHECK_LAUNCH();
-            PRC_TRY(R.vcycle(l, R.B[l].v, R.B[l].f, true));
-            PRC_LAUNCH_B("mg_correct_fp64", st, 20.0 * N,
-                         launch_pdl(add_kernel<double, float>, grid_for(N), 256, 0, st, m.v64[l], R.B[l].v, N));
-            PRC_CHECK_LAUNCH();
+            PRC_TRY(R.vcycle(l, R.B[l].v, R.B[l].f, true, m.v64[l]));
         }
     }
     return PRC_OK;
@@ -1523,9 +1688,12 @@ prc_status_t prc_multigrid_f64(const double* delta, double* phi, const int32_t n
         int n[3] = {nmesh[0], nmesh[1], nmesh[2]};                                                                   \
         Stencil<T> s = make_stencil<T>(n, boxsize, boxcenter, beta, los);                                            \
         const double bytes = 3.0 * sizeof(T) * n[0] * n[1] * n[2];                                                   \
-        if (quad_ok(n, v, f, r))                                                                                     \
+        if (quad_ok(n, v, f, r) && march_ok(s, 1))                                                             \
             PRC_LAUNCH_B("mg_residual", (cudaStream_t)stream, bytes,                                                 \
-                         residual4_kernel<T, T, T, T, T>(mg_mode(s))                                              \
+                         (launch_march<T, T, OP_RESIDUAL>(v, f, r, nullptr, s, (T)0, 1, (cudaStream_t)stream)));   \
+        else if (quad_ok(n, v, f, r))                                                                                     \
+            PRC_LAUNCH_B("mg_residual", (cudaStream_t)stream, bytes,                                                 \
+                         residual4_kernel<T, T>(mg_mode(s))                                              \
                              <<<grid3_quad(n).grid, grid3_quad(n).block, 0, (cudaStream_t)stream>>>(v, f, r, s));     \
         else                                                                                                         \
             PRC_LAUNCH_B("mg_residual", (cudaStream_t)stream, bytes,                                                 \
@@ -1536,17 +1704,17 @@ prc_status_t prc_multigrid_f64(const double* delta, double* phi, const int32_t n
     }                                                                                                                \
     prc_status_t prc_mg_reduce_##SUF(const T* fine, T* coarse, const int32_t nf[3], void* stream) {                 \
         if (!fine || !coarse || !nf) return PRC_ERR_ARG;                                                             \
-        Dims d = {{nf[0], nf[1], nf[2]}};                                                                            \
+        const int n[3] = {nf[0], nf[1], nf[2]};                                                                       \
         PRC_LAUNCH("mg_reduce", (cudaStream_t)stream,                                                                \
-                   reduce_kernel<T, T, T><<<grid3_coarse(nf).grid, grid3_coarse(nf).block, 0, (cudaStream_t)stream>>>(fine, coarse, d)); \
+                   launch_reduce(fine, coarse, n, 1, (cudaStream_t)stream)); \
         PRC_CHECK_LAUNCH();                                                                                          \
         return PRC_OK;                                                                                               \
     }                                                                                                                \
     prc_status_t prc_mg_prolong_##SUF(const T* coarse, T* fine, const int32_t nc[3], void* stream) {                \
         if (!fine || !coarse || !nc) return PRC_ERR_ARG;                                                             \
-        Dims d = {{nc[0], nc[1], nc[2]}};                                                                            \
+        const int n[3] = {nc[0], nc[1], nc[2]};                                                                       \
         PRC_LAUNCH("mg_prolong", (cudaStream_t)stream,                                                               \
-                   prolong_kernel<T, T, T, false><<<grid3(nc).grid, grid3(nc).block, 0, (cudaStream_t)stream>>>(coarse, fine, d)); \
+                   (launch_prolong<T, false>(coarse, fine, n, 1, (cudaStream_t)stream))); \
         PRC_CHECK_LAUNCH();                                                                                          \
         return PRC_OK;                                                                                               \
     }
