@@ -174,6 +174,26 @@ inline cudaError_t launch_pdl(void (*kernel)(K...), dim3 grid, dim3 block, size_
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<K>(args)...);
 }
 
+// The same with the grid in clusters of `cluster` blocks along x.
+template <typename... K, typename... A>
+inline cudaError_t launch_cluster_pdl(void (*kernel)(K...), dim3 grid, dim3 block, int cluster, size_t smem,
+                                      cudaStream_t st, A&&... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = cluster;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = pdl_enabled() ? 2 : 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<K>(args)...);
+}
+
 // Adds n to the launch counter (kernels replayed inside a CUDA graph launch).
 void add_launches(unsigned long long n);
 // Launches and compulsory bytes recorded by this thread's captures since the last call (reset).

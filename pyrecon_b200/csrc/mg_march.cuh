@@ -57,6 +57,13 @@ template <bool LOCAL, typename A> __device__ __forceinline__ A z_p2(const OpCoef
     return LOCAL ? rn_add(rn_add((A)(z & ~3), k.off2), (A)(z & 3)) : k.off2;
 }
 
+// FP32: the hardware reciprocal (1 ulp; its argument is a sum of squares of cell numbers, far from the subnormals).
+__device__ __forceinline__ float rcp_approx(float a) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a));
+    return r;
+}
+
 // ---- two cells at once ----
 // FP32 pairs go through the packed instructions (one issue slot for two cells, the same rounding per cell; a 512^3
 // sweep 330 us against 350 with scalar ones), FP64 pairs through two scalar ones.
@@ -64,6 +71,9 @@ template <typename A> struct Pair;
 template <> struct Pair<float> {
     typedef float2 T;
     static __device__ __forceinline__ T make(float a, float b) { return make_float2(a, b); }
+    static __device__ __forceinline__ T all(float a) { return make_float2(a, a); }
+    static __device__ __forceinline__ T div_sub(T a, T b, T c) { return fma(a, make(rcp_approx(b.x), rcp_approx(b.y)), make(-c.x, -c.y)); }
+    static __device__ __forceinline__ T div(float a, T b) { return mul(all(a), make(rcp_approx(b.x), rcp_approx(b.y))); }
     static __device__ __forceinline__ T add(T a, T b) { return __fadd2_rn(a, b); }
     static __device__ __forceinline__ T sub(T a, T b) { return __ffma2_rn(b, make_float2(-1.f, -1.f), a); }
     static __device__ __forceinline__ T mul(T a, T b) { return __fmul2_rn(a, b); }
@@ -72,74 +82,74 @@ template <> struct Pair<float> {
 template <> struct Pair<double> {
     typedef double2 T;
     static __device__ __forceinline__ T make(double a, double b) { return make_double2(a, b); }
+    static __device__ __forceinline__ T all(double a) { return make_double2(a, a); }
+    static __device__ __forceinline__ T div_sub(T a, T b, T c) { return sub(make(a.x / b.x, a.y / b.y), c); }
+    static __device__ __forceinline__ T div(double a, T b) { return make(a / b.x, a / b.y); }
     static __device__ __forceinline__ T add(T a, T b) { return make(rn_add(a.x, b.x), rn_add(a.y, b.y)); }
     static __device__ __forceinline__ T sub(T a, T b) { return make(rn_sub(a.x, b.x), rn_sub(a.y, b.y)); }
     static __device__ __forceinline__ T mul(T a, T b) { return make(rn_mul(a.x, b.x), rn_mul(a.y, b.y)); }
     static __device__ __forceinline__ T fma(T a, T b, T c) { return make(fma_rn(a.x, b.x, c.x), fma_rn(a.y, b.y, c.y)); }
 };
+// One cell, with the same operations.
+template <typename A> struct One {
+    typedef A T;
+    static __device__ __forceinline__ A all(A a) { return a; }
+    static __device__ __forceinline__ A add(A a, A b) { return rn_add(a, b); }
+    static __device__ __forceinline__ A sub(A a, A b) { return rn_sub(a, b); }
+    static __device__ __forceinline__ A mul(A a, A b) { return rn_mul(a, b); }
+    static __device__ __forceinline__ A fma(A a, A b, A c) { return fma_rn(a, b, c); }
+    static __device__ __forceinline__ A div_sub(A a, A b, A c) {
+        if constexpr (sizeof(A) == 4) return fma_rn(a, rcp_approx(b), -c);
+        else return rn_sub(a / b, c);
+    }
+    static __device__ __forceinline__ A div(A a, A b) {
+        if constexpr (sizeof(A) == 4) return rn_mul(a, rcp_approx(b));
+        else return a / b;
+    }
+};
 template <typename A> __device__ __forceinline__ typename Pair<A>::T both(A a) { return Pair<A>::make(a, a); }
 
-// U, W, q and P of two cells from their neighbours (xp .. zm) and edge sums e_ab.
-template <bool LOCAL, typename A, typename P2 = typename Pair<A>::T>
-__device__ __forceinline__ void op_terms(const OpCoef<A>& k, const XYCoef<A>& c, P2 p2, P2 s2, P2 xp, P2 xm, P2 yp, P2 ym,
-                                         P2 zp, P2 zm, P2 exy, P2 exz, P2 eyz, P2& U, P2& W, P2& q, P2& PP) {
-    typedef Pair<A> P;
-    const P2 Sx = P::add(xp, xm), Sy = P::add(yp, ym), Sz = P::add(zp, zm);
-    U = P::fma(both(k.ih0), Sx, P::mul(both(k.ih1), Sy));
-    U = P::fma(both(k.ih2), Sz, U);
+// U, W, q and P of the cells of ops O from their neighbours (xp .. zm) and edge sums e_ab.
+template <bool LOCAL, typename O, typename A, typename V = typename O::T>
+__device__ __forceinline__ void op_terms(const OpCoef<A>& k, const XYCoef<A>& c, V p2, V s2, V xp, V xm, V yp, V ym, V zp,
+                                         V zm, V exy, V exz, V eyz, V& U, V& W, V& q, V& PP) {
+    const V Sx = O::add(xp, xm), Sy = O::add(yp, ym), Sz = O::add(zp, zm);
+    U = O::fma(O::all(k.ih0), Sx, O::mul(O::all(k.ih1), Sy));
+    U = O::fma(O::all(k.ih2), Sz, U);
     if (LOCAL) {
-        W = P::fma(both(c.ap), xp, P::mul(both(c.am), xm));
-        W = P::fma(both(c.bp), yp, W);
-        W = P::fma(both(c.bm), ym, W);
-        W = P::fma(P::add(s2, p2), zp, W);
-        W = P::fma(P::sub(s2, p2), zm, W);
+        W = O::fma(O::all(c.ap), xp, O::mul(O::all(c.am), xm));
+        W = O::fma(O::all(c.bp), yp, W);
+        W = O::fma(O::all(c.bm), ym, W);
+        W = O::fma(O::add(s2, p2), zp, W);
+        W = O::fma(O::sub(s2, p2), zm, W);
     } else {
-        W = P::fma(both(c.s0), Sx, P::mul(both(c.s1), Sy));
-        W = P::fma(s2, Sz, W);
+        W = O::fma(O::all(c.s0), Sx, O::mul(O::all(c.s1), Sy));
+        W = O::fma(s2, Sz, W);
     }
-    W = P::fma(both(c.e01), exy, W);
-    W = P::fma(P::mul(both(c.hp0), p2), exz, W);
-    W = P::fma(P::mul(both(c.hp1), p2), eyz, W);
-    q = P::fma(both(k.h22), s2, both(c.q01));
-    PP = P::add(both(c.P01), s2);
+    W = O::fma(O::all(c.e01), exy, W);
+    W = O::fma(O::mul(O::all(c.hp0), p2), exz, W);
+    W = O::fma(O::mul(O::all(c.hp1), p2), eyz, W);
+    q = O::fma(O::all(k.h22), s2, O::all(c.q01));
+    PP = O::add(O::all(c.P01), s2);
 }
 
-__device__ __forceinline__ float2 neg2(float2 a) { return make_float2(-a.x, -a.y); }
-__device__ __forceinline__ double2 neg2(double2 a) { return make_double2(-a.x, -a.y); }
-
-// FP32: the hardware reciprocal (1 ulp; its argument is a sum of squares of cell numbers, far from the subnormals).
-__device__ __forceinline__ float rcp_approx(float a) {
-    float r;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a));
-    return r;
+// The damped-Jacobi values v + w (num / den - v).
+template <typename O, typename A, typename V = typename O::T>
+__device__ __forceinline__ V op_jacobi(const OpCoef<A>& k, V f, V v, V U, V W, V q, V PP, A w) {
+    const V num = O::fma(q, O::add(f, U), O::mul(O::all(k.beta), W));
+    const V den = O::fma(q, O::all(k.sih2), O::mul(O::all(k.beta2), PP));
+    return O::fma(O::all(w), O::div_sub(num, den, v), v);
 }
 
-// The damped-Jacobi values v + w (num / den - v) of two cells.
-template <typename A, typename P2 = typename Pair<A>::T>
-__device__ __forceinline__ P2 op_jacobi(const OpCoef<A>& k, P2 f, P2 v, P2 U, P2 W, P2 q, P2 PP, A w) {
-    typedef Pair<A> P;
-    const P2 num = P::fma(q, P::add(f, U), P::mul(both(k.beta), W));
-    const P2 den = P::fma(q, both(k.sih2), P::mul(both(k.beta2), PP));
-    P2 t;
-    if constexpr (sizeof(A) == 4) t = P::fma(num, P::make(rcp_approx(den.x), rcp_approx(den.y)), neg2(v));
-    else t = P::sub(P::make(num.x / den.x, num.y / den.y), v);
-    return P::fma(both(w), t, v);
+// f - A v; t2 = W - 2 P v.
+template <typename O, typename A, typename V = typename O::T>
+__device__ __forceinline__ V op_residual_from(const OpCoef<A>& k, V f, V v, V U, V t2, V q) {
+    const V t1 = O::fma(O::all(-k.sih2), v, O::add(f, U));
+    return O::fma(O::div(k.beta, q), t2, t1);
 }
-
-// f - A v of two cells; t2 = W - 2 P v.
-template <typename A, typename P2 = typename Pair<A>::T>
-__device__ __forceinline__ P2 op_residual_from(const OpCoef<A>& k, P2 f, P2 v, P2 U, P2 t2, P2 q) {
-    typedef Pair<A> P;
-    P2 g;
-    if constexpr (sizeof(A) == 4) g = P::mul(both(k.beta), P::make(rcp_approx(q.x), rcp_approx(q.y)));
-    else g = P::make(k.beta / q.x, k.beta / q.y);
-    const P2 t1 = P::fma(both(-k.sih2), v, P::add(f, U));
-    return P::fma(g, t2, t1);
-}
-template <typename A, typename P2 = typename Pair<A>::T>
-__device__ __forceinline__ P2 op_residual(const OpCoef<A>& k, P2 f, P2 v, P2 U, P2 W, P2 q, P2 PP) {
-    typedef Pair<A> P;
-    return op_residual_from(k, f, v, U, P::fma(P::mul(both((A)-2), PP), v, W), q);
+template <typename O, typename A, typename V = typename O::T>
+__device__ __forceinline__ V op_residual(const OpCoef<A>& k, V f, V v, V U, V W, V q, V PP) {
+    return op_residual_from<O>(k, f, v, U, O::fma(O::mul(O::all((A)-2), PP), v, W), q);
 }
 
 // ---- the march ----
@@ -341,10 +351,10 @@ __global__ void __launch_bounds__(MARCH_THREADS, 2)
                 const P2 eyz = P::make(rn_sub(rn_add(Yp[u][j].y, yml), rn_add(Ym[u][j].y, ypl)),
                                        rn_sub(rn_add(ypr, Ym[u][j].x), rn_add(ymr, Yp[u][j].x)));
                 P2 U, W, q, PP;
-                op_terms<LOCAL>(k, c, p2[j], s2[j], C[ip][j], C[im][j], Yp[u][j], Ym[u][j], zp, zm, exy, exz, eyz, U, W, q,
+                op_terms<LOCAL, P>(k, c, p2[j], s2[j], C[ip][j], C[im][j], Yp[u][j], Ym[u][j], zp, zm, exy, exz, eyz, U, W, q,
                                 PP);
-                const P2 r = OP == OP_RESIDUAL ? op_residual(k, fv[j], C[u][j], U, W, q, PP)
-                                               : op_jacobi(k, fv[j], C[u][j], U, W, q, PP, w);
+                const P2 r = OP == OP_RESIDUAL ? op_residual<P>(k, fv[j], C[u][j], U, W, q, PP)
+                                               : op_jacobi<P>(k, fv[j], C[u][j], U, W, q, PP, w);
                 o[2 * j] = r.x, o[2 * j + 1] = r.y;
             }
             if (mine && x >= x_own) {

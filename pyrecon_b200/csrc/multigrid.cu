@@ -268,7 +268,7 @@ __device__ __forceinline__ void quad_terms(const QuadCols<T>& Q, const OpCoef<T>
                               P::add(P::make(Q.XM[i + 2], Q.XM[i + 3]), P::make(Q.XP[i], Q.XP[i + 1])));
         const P2 eyz = P::sub(P::add(P::make(Q.YP[i + 2], Q.YP[i + 3]), P::make(Q.YM[i], Q.YM[i + 1])),
                               P::add(P::make(Q.YM[i + 2], Q.YM[i + 3]), P::make(Q.YP[i], Q.YP[i + 1])));
-        op_terms<LOCAL>(k, c, p2, s2, xp, xm, yp, ym, zp, zm, exy, exz, eyz, U, W, q, PP);
+        op_terms<LOCAL, P>(k, c, p2, s2, xp, xm, yp, ym, zp, zm, exy, exz, eyz, U, W, q, PP);
     }
 }
 
@@ -283,7 +283,7 @@ __device__ __forceinline__ void quad_jacobi(const QuadCols<T>& Q, const OpCoef<T
         typename P::T U, W, wf, q, PP;
         quad_terms<MODE>(Q, k, c, z0, j, U, W, wf, q, PP);
         if (MODE >= MG_AXIS0) W = P::mul(wf, W);
-        const typename P::T r = op_jacobi(k, P::make(f[2 * j], f[2 * j + 1]), P::make(Q.c[2 * j + 1], Q.c[2 * j + 2]), U, W,
+        const typename P::T r = op_jacobi<P>(k, P::make(f[2 * j], f[2 * j + 1]), P::make(Q.c[2 * j + 1], Q.c[2 * j + 2]), U, W,
                                           q, PP, w);
         o[2 * j] = r.x, o[2 * j + 1] = r.y;
     }
@@ -306,7 +306,7 @@ __device__ __forceinline__ void quad_zero(const OpCoef<T>& k, T w, int x, int y,
     for (int j = 0; j < 2; j++) {
         const P2 p2 = LOCAL ? P::make(rn_add((T)(z0 + 2 * j), k.off2), rn_add((T)(z0 + 2 * j + 1), k.off2)) : both(k.off2);
         const P2 s2 = P::mul(p2, p2), q = P::fma(both(k.h22), s2, both(c.q01)), PP = P::add(both(c.P01), s2);
-        const P2 r = op_jacobi(k, P::make(f[2 * j], f[2 * j + 1]), zero, zero, zero, q, PP, w);
+        const P2 r = op_jacobi<P>(k, P::make(f[2 * j], f[2 * j + 1]), zero, zero, zero, q, PP, w);
         o[2 * j] = r.x, o[2 * j + 1] = r.y;
     }
 }
@@ -541,10 +541,10 @@ __global__ void __launch_bounds__(256) residual_kernel4(const A* __restrict__ v,
         const typename P::T v2 = P::make(Q.c[2 * j + 1], Q.c[2 * j + 2]), f2 = P::make(fv[2 * j], fv[2 * j + 1]);
         typename P::T t;
         if constexpr (MODE >= MG_AXIS0 && sizeof(A) == 4) {
-            t = op_residual_from(k, f2, v2, U, P::fma(wf, W, P::mul(P::mul(both((A)-2), PP), v2)), qq);
+            t = op_residual_from<P>(k, f2, v2, U, P::fma(wf, W, P::mul(P::mul(both((A)-2), PP), v2)), qq);
         } else {
             if (MODE >= MG_AXIS0) W = P::mul(wf, W);
-            t = op_residual(k, f2, v2, U, W, qq, PP);
+            t = op_residual<P>(k, f2, v2, U, W, qq, PP);
         }
         o[2 * j] = (R)t.x, o[2 * j + 1] = (R)t.y;
     }
@@ -879,30 +879,6 @@ static int mg_tb_default(const int n[3], size_t tsize) {
     return 0;
 }
 
-// ---- the V-cycle of the smallest levels in one block per problem ----
-// Below a few thousand cells a level costs more in launches than in work: a V-cycle visit of the levels
-// under 16^3 is ~40 kernels of a few microseconds each.  vcycle_small runs the V-cycle of levels
-// l0 .. l0 + nl - 1 (MGRunner::vcycle's pre-sweeps, residual, restriction, prolongation and post-sweeps,
-// with the one-cell expressions of jacobi_sweep, residual_kernel, reduce_kernel and prolong_kernel) in one
-// block, each level's v, f and scratch in shared memory, a block barrier between steps.  The problems of
-// a batch are one block each.
-constexpr int MG_SMALL_LEVELS = 8;
-constexpr int MG_SMALL_THREADS = 512;
-// Default top level of vcycle_small: 8^3.  Measured per 256^3 local-line-of-sight solve, 10.40 ms with every
-// step its own graph node, 10.05 ms from 8^3 down, 11.98 ms from 16^3 down (one block then does ~93k cell
-// updates per visit on one SM, slower than the ~40 launches it replaces).
-constexpr int MG_SMALL_DEFAULT_CELLS = 512;
-constexpr size_t MG_SMALL_MAX_SMEM = 200 * 1024;
-
-template <typename T> struct SmallVCycle {
-    int nl;
-    Stencil<T> s[MG_SMALL_LEVELS];
-    int off[MG_SMALL_LEVELS];    // level l's arrays v, f, scratch (cells(l) values each) start at off[l]
-    T w;
-    int jn;
-    int zero_v;                  // the top level's v starts at zero (not read)
-};
-
 __device__ __forceinline__ int cells_of(const int n[3]) { return n[0] * n[1] * n[2]; }
 
 __device__ __forceinline__ void cell_xyz(int i, const int n[3], int& x, int& y, int& z) {
@@ -911,136 +887,11 @@ __device__ __forceinline__ void cell_xyz(int i, const int n[3], int& x, int& y, 
     x = i / (n[1] * n[2]);
 }
 
-template <typename T>
-__device__ void small_sweeps(const Stencil<T>& s, T*& v, const T* f, T*& tmp, T w, int niter, bool zero) {
-    const int N = cells_of(s.n);
-    if (niter == 0 && zero)
-        for (int i = threadIdx.x; i < N; i += blockDim.x) v[i] = (T)0;
-    for (int it = 0; it < niter; it++) {
-        const bool z0 = zero && it == 0;
-        for (int i = threadIdx.x; i < N; i += blockDim.x) {
-            int x, y, z;
-            cell_xyz(i, s.n, x, y, z);
-            T p[3], g, G[3];
-            coeffs<T>(s, x, y, z, p, g, G);
-            T jac = f[i];
-            T vc = (T)0;
-            if (!z0) {
-                jac += neighbour_sum<T, T, true>(v, s.n, x, y, z, p, g, G, s.local);
-                vc = v[i];
-            }
-            jac /= (T)2 * (G[0] + G[1] + G[2]);
-            tmp[i] = ((T)1 - w) * vc + w * jac;
-        }
-        T* t = v;
-        v = tmp;
-        tmp = t;
-        __syncthreads();
-    }
-    __syncthreads();
-}
+}  // namespace prc
 
-template <typename T>
-__global__ void __launch_bounds__(MG_SMALL_THREADS) vcycle_small(const T* __restrict__ fg, T* __restrict__ vg,
-                                                                 SmallVCycle<T> P) {
-    pdl_trigger();
-    pdl_wait();
-    extern __shared__ __align__(16) unsigned char mg_smem[];
-    T* sm = (T*)mg_smem;
-    const int N0 = cells_of(P.s[0].n);
-    fg += (int64_t)blockIdx.x * N0;
-    vg += (int64_t)blockIdx.x * N0;
-    T *v[MG_SMALL_LEVELS], *f[MG_SMALL_LEVELS], *t[MG_SMALL_LEVELS];
-    for (int l = 0; l < P.nl; l++) {
-        const int N = cells_of(P.s[l].n);
-        v[l] = sm + P.off[l];
-        f[l] = v[l] + N;
-        t[l] = f[l] + N;
-    }
-    for (int i = threadIdx.x; i < N0; i += blockDim.x) {
-        f[0][i] = fg[i];
-        if (!P.zero_v) v[0][i] = vg[i];
-    }
-    __syncthreads();
-    // down: pre-sweeps, then the residual restricted to the next level's right-hand side
-    for (int l = 0; l < P.nl; l++) {
-        const Stencil<T>& s = P.s[l];
-        small_sweeps(s, v[l], f[l], t[l], P.w, P.jn, l > 0 || P.zero_v);
-        if (l + 1 == P.nl) break;
-        const int N = cells_of(s.n);
-        for (int i = threadIdx.x; i < N; i += blockDim.x) {
-            int x, y, z;
-            cell_xyz(i, s.n, x, y, z);
-            T p[3], g, G[3];
-            coeffs<T>(s, x, y, z, p, g, G);
-            const T nb = neighbour_sum<T, T, true>(v[l], s.n, x, y, z, p, g, G, s.local);
-            const T av = (T)2 * (G[0] + G[1] + G[2]) * v[l][i] - nb;
-            t[l][i] = f[l][i] - av;
-        }
-        __syncthreads();
-        const int* nf = s.n;
-        const int* nc = P.s[l + 1].n;
-        const int Nc = cells_of(nc);
-        for (int i = threadIdx.x; i < Nc; i += blockDim.x) {
-            int x, y, z;
-            cell_xyz(i, nc, x, y, z);
-            const int X[3] = {wrap_dn(2 * x, nf[0]), 2 * x, wrap_up(2 * x, nf[0])};
-            const int Y[3] = {wrap_dn(2 * y, nf[1]), 2 * y, wrap_up(2 * y, nf[1])};
-            const int Z[3] = {wrap_dn(2 * z, nf[2]), 2 * z, wrap_up(2 * z, nf[2])};
-            T acc = 0;
-#pragma unroll
-            for (int a = 0; a < 3; a++)
-#pragma unroll
-                for (int b = 0; b < 3; b++) {
-                    const T* row = t[l] + (X[a] * nf[1] + Y[b]) * nf[2];
-#pragma unroll
-                    for (int c = 0; c < 3; c++) {
-                        const int side = (a != 1) + (b != 1) + (c != 1);
-                        acc += (T)(8 >> side) * row[Z[c]];
-                    }
-                }
-            f[l + 1][i] = acc / (T)64;
-        }
-        __syncthreads();
-    }
-    // up: the coarse correction prolonged and added, then post-sweeps
-    for (int l = P.nl - 1; l >= 0; l--) {
-        if (l + 1 < P.nl) {
-            const int* nc = P.s[l + 1].n;
-            const int Nc = cells_of(nc);
-            const int nf1 = 2 * nc[1], nf2 = 2 * nc[2];
-            for (int i = threadIdx.x; i < Nc; i += blockDim.x) {
-                int x, y, z;
-                cell_xyz(i, nc, x, y, z);
-                const int xs[2] = {x, wrap_up(x, nc[0])}, ys[2] = {y, wrap_up(y, nc[1])}, zs[2] = {z, wrap_up(z, nc[2])};
-                T c[2][2][2];
-#pragma unroll
-                for (int a = 0; a < 2; a++)
-#pragma unroll
-                    for (int b = 0; b < 2; b++)
-#pragma unroll
-                        for (int d = 0; d < 2; d++) c[a][b][d] = v[l + 1][(xs[a] * nc[1] + ys[b]) * nc[2] + zs[d]];
-#pragma unroll
-                for (int e = 0; e < 8; e++) {
-                    const int ex = (e >> 2) & 1, ey = (e >> 1) & 1, ez = e & 1;
-                    T sum = 0;
-#pragma unroll
-                    for (int a = 0; a <= ex; a++)
-#pragma unroll
-                        for (int b = 0; b <= ey; b++)
-#pragma unroll
-                            for (int d = 0; d <= ez; d++) sum += c[a][b][d];
-                    sum /= (T)((1 + ex) * (1 + ey) * (1 + ez));
-                    T* dst = v[l] + ((2 * x + ex) * nf1 + (2 * y + ey)) * nf2 + (2 * z + ez);
-                    *dst = *dst + sum;
-                }
-            }
-            __syncthreads();
-        }
-        small_sweeps(P.s[l], v[l], f[l], t[l], P.w, P.jn, false);
-    }
-    for (int i = threadIdx.x; i < N0; i += blockDim.x) vg[i] = v[0][i];
-}
+#include "mg_coarse.cuh"
+
+namespace prc {
 
 // ---------------------------------------------------------------------------------------------
 // Level hierarchy and the FMG / V-cycle drivers
@@ -1150,31 +1001,47 @@ template <typename T> struct MGRunner {
         return PRC_OK;
     }
 
-    // The V-cycle from level l down as one vcycle_small launch, when level l has at most "mg_small_cells"
+    // The V-cycle from level l down as one vcycle_coarse launch, when level l has at most "mg_small_cells"
     // cells (run-time knob, key 0; 0 runs every step as its own kernel) and its levels fit in shared memory.
-    int small_vcycle(int l, T* v, const T* f, bool v_zero, bool* done) {
+    int coarse_vcycle(int l, T* v, const T* f, bool v_zero, bool* done) {
         *done = false;
-        const int limit = tune_get("mg_small_cells", 0, MG_SMALL_DEFAULT_CELLS);
+        const int limit = tune_get("mg_small_cells", 0, MG_COARSE_DEFAULT_CELLS);
         const int nl = (int)L.size() - l;
-        if (limit <= 0 || L[l].size() > limit || nl > MG_SMALL_LEVELS) return PRC_OK;
-        SmallVCycle<T> sv;
-        size_t off = 0;
-        sv.nl = nl;
+        if (limit <= 0 || L[l].size() > limit || nl > MG_COARSE_LEVELS) return PRC_OK;
+        CoarseCycle<T> c;
+        c.nl = nl;
+        c.ndist = 0;
+        // rows of four cells are dealt (the quad kernels' arithmetic, by pairs); the rest stays in block 0
+        const int slots = MG_COARSE_SLOTS * MG_COARSE_THREADS;
+        while (c.ndist < nl && L[l + c.ndist].size() > MG_SINGLE_CELLS && L[l + c.ndist].n[2] % 4 == 0) c.ndist++;
+        if (c.ndist < nl && L[l + c.ndist].size() > slots) return PRC_OK;
+        c.base = c.ndist > 0 ? L[l + c.ndist - 1].n[0] : 0;
+        int cl = 1;
+        while (c.ndist > 0 && 2 * cl <= std::min(c.base, MG_COARSE_CLUSTER)) cl *= 2;
+        if (c.ndist > 0 &&
+            ((int64_t)((c.base + cl - 1) / cl) << (c.ndist - 1)) * L[l].n[1] * (L[l].n[2] / 2) > slots)
+            return PRC_OK;
+        size_t at = 0;
         for (int j = 0; j < nl; j++) {
-            sv.s[j] = stencil(l + j);
-            sv.off[j] = (int)off;
-            off = (off + 3 * (size_t)L[l + j].size() + 3) & ~(size_t)3;
+            const Level& lv = L[l + j];
+            c.s[j] = stencil(l + j);
+            const int64_t planes = j < c.ndist ? (int64_t)((c.base + cl - 1) / cl) << (c.ndist - 1 - j) : lv.n[0];
+            const int64_t pl = (int64_t)lv.n[1] * lv.n[2], own = (planes * pl + 3) & ~3ll;
+            c.vsize[j] = (int)(((planes + (j < c.ndist ? 2 : 0)) * pl + 3) & ~3ll);
+            c.at[j] = (int)at;
+            at += 2 * (size_t)c.vsize[j] + own;
+            if (at * sizeof(T) > MG_COARSE_MAX_SMEM) return PRC_OK;
         }
-        const size_t smem = off * sizeof(T);
-        if (smem > MG_SMALL_MAX_SMEM) return PRC_OK;
-        sv.w = (T)P.damping;
-        sv.jn = P.jn;
-        sv.zero_v = v_zero ? 1 : 0;
-        if (smem > 48 * 1024 &&
-            cudaFuncSetAttribute(vcycle_small<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+        const size_t smem = at * sizeof(T);
+        c.w = (T)P.damping;
+        c.jn = P.jn;
+        c.zero_v = v_zero ? 1 : 0;
+        c.axis = mg_mode(c.s[0]) >= MG_AXIS0 ? mg_mode(c.s[0]) - MG_AXIS0 : -1;
+        const auto kernel = c.s[0].local ? vcycle_coarse<T, true> : vcycle_coarse<T, false>;
+        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MG_COARSE_MAX_SMEM) != cudaSuccess)
             return PRC_ERR_CUDA;
-        PRC_LAUNCH_B("mg_vcycle_small", st, (double)L[l].size() * count * sizeof(T) * (v_zero ? 2 : 3),
-                     launch_pdl(vcycle_small<T>, dim3(count), dim3(MG_SMALL_THREADS), smem, st, f, v, sv));
+        PRC_LAUNCH_B("mg_vcycle_coarse", st, (double)L[l].size() * count * sizeof(T) * (v_zero ? 2 : 3),
+                     launch_cluster_pdl(kernel, dim3(cl * count), dim3(MG_COARSE_THREADS), cl, smem, st, f, v, c));
         PRC_CHECK_LAUNCH();
         *done = true;
         return PRC_OK;
@@ -1184,7 +1051,7 @@ template <typename T> struct MGRunner {
     // acc (optional): the cycle's result is added to it; where the last step could do so itself, v holds nothing.
     int vcycle(int l, T*& v, const T* f, bool v_zero, double* acc = nullptr) {
         bool small = false;
-        PRC_TRY(small_vcycle(l, v, f, v_zero, &small));
+        PRC_TRY(coarse_vcycle(l, v, f, v_zero, &small));
         if (small || P.jn == 0) {
             if (!small) PRC_TRY(vcycle_steps(l, v, f, v_zero, nullptr));
             if (acc != nullptr) {

@@ -76,3 +76,46 @@ def test_batched_solve_crossing_to_the_march(dtype):
     for d, phi in zip(deltas, together):
         assert np.isfinite(phi).all()
         np.testing.assert_array_equal(phi, solve([d])[0])
+
+
+@pytest.mark.parametrize('dtype', ['f4', 'f8'])
+@pytest.mark.parametrize('nmesh,los', [((40, 48, 32), None), ((80, 40, 56), [0.3, -0.5, 0.8]), ((24, 64, 96), [1., 0., 0.]),
+                                       ((20, 12, 24), None), ((12, 12, 28), [0., 0., 1.]), ((96, 24, 12), None)])
+def test_coarse_levels_dealt_over_a_cluster(dtype, nmesh, los):
+    """V-cycles of the coarse levels in one kernel (planes dealt unevenly, levels that stay in one block, rows of four and of
+    two) against every step launched by itself (mg_small_cells = 0), for one problem and two."""
+    import torch as t
+    from pyrecon_b200 import _lib as L
+    lib, st = L.load(), L.stream_of(t.device('cuda', 0))
+    mixed = int(dtype == 'f4')
+    td = t.float32 if mixed else t.float64
+    gen = t.Generator(device='cuda').manual_seed(6)
+    deltas = [t.randn(nmesh, generator=gen, device='cuda', dtype=td) for _ in range(2)]
+    if los is not None:
+        los = list(np.asarray(los) / np.linalg.norm(los))
+    tail = [L.i3(nmesh), L.d3([800., 700., 900.]), L.d3([1500.] * 3), 0.4, 0.4, 5, 6, L.opt_d3(los)]
+
+    def solve(ds):
+        n = len(ds)
+        ws = t.empty(lib.prc_multigrid_batch_workspace_bytes(L.i3(nmesh), 4 if mixed else 8, mixed, n), dtype=t.uint8,
+                     device='cuda')
+        phis = [t.empty_like(d) for d in ds]
+        L.call('prc_multigrid_batch_' + L.suffix(dtype), L.pointer_array(ds), L.pointer_array(phis), n, *tail,
+               *([1] if mixed else []), L.ptr(ws), ws.numel(), st)
+        t.cuda.synchronize()
+        return [x.cpu().numpy() for x in phis]
+
+    n0 = L.launch_count()
+    fused = solve(deltas)
+    n1 = L.launch_count()
+    np.testing.assert_array_equal(fused[1], solve(deltas[1:])[0])
+    L.tune_set('mg_small_cells', 0, 0)
+    try:
+        n2 = L.launch_count()
+        steps = solve(deltas)
+        assert L.launch_count() - n2 > n1 - n0
+    finally:
+        L.tune_set('mg_small_cells', 0, -1)
+    for a, b in zip(fused, steps):
+        assert np.isfinite(a).all()
+        assert maxrel(a, b) < (1e-5 if dtype == 'f4' else 1e-12)
