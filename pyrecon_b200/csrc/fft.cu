@@ -26,6 +26,7 @@
 #include <algorithm>
 #include <map>
 #include <mutex>
+#include <type_traits>
 #include <math.h>
 #include <string.h>
 #include <stdlib.h>
@@ -709,6 +710,7 @@ __global__ void debug_wait_timeout(uint64_t limit_ns, uint32_t bytes, int* out) 
 
 #include "fft_fast.cuh"
 #include "fft_tma.cuh"
+#include "fft_duo.cuh"
 
 // ---------------------------------------------------------------------------------------------
 // Host-side planning and launches
@@ -1028,25 +1030,53 @@ template <typename T, int N> struct StridedTmaCfg {
     static constexpr size_t SMEM = fast::TmaSmem<T, N, B, S, fast::StridedPP<T, N, B, S>::value ? 1 : 0>::BYTES;
 };
 
+// Pairs of columns a tile and blocks an SM of the FP32 passes on pairs of columns (fft_duo.cuh): about 16 warps an SM
+// (128 registers a thread).  Strided tiles have 128-byte rows where they fit; the k-space and Hessian passes 64-byte rows,
+// so that several blocks share an SM and a small mesh has tiles for all of them (k-space launch at 256: 0.100 ms against
+// 0.106 with 128-byte rows, at 128: 0.018 against 0.022).  They run where they are faster and keep the results to the
+// bit: strided and Hessian passes of 64 to 1024 points without a radix-3 step (y forward at 512 x 512 x 257: 0.282 ms a
+// pass with one column a thread, 0.237 with two; y inverse 0.288 and 0.244, Hessian 1.267 and 1.053; forward at 256: 0.058
+// and 0.044, at 128: 0.013 and 0.011), k-space passes of up to 512 points (512, three outputs: 0.88 and 0.70; 256: 0.109
+// and 0.100; 128: 0.017 and 0.018, but 0.022 with one column behind a y pass with two, whose shared-memory split of the
+// SM differs) of the four operators below.  Lines of 3 2^k points, 1024-point k-space lines and the one-output iteration
+// along a fixed line of sight round elsewhere in their chains of products and sums, and keep one column a thread.
+template <int N> struct DuoCfg {
+    static constexpr bool OK = N >= 64 && N % 3 != 0, K_OK = OK && N <= 512;
+    static constexpr int KBP = 4, SBP = N >= 1024 ? 4 : 8, S = 2;
+    static constexpr int KTHREADS = N / 8 * KBP, STHREADS = N / 8 * SBP;
+    static constexpr size_t KSMEM = fast::KSpaceDuoSmem<N, KBP>::BYTES, SSMEM = fast::StridedDuoSmem<N, SBP, S>::BYTES;
+    static constexpr size_t HSMEM = fast::HessDuoSmem<N, KBP, S>::BYTES;
+    static constexpr int fit(size_t smem, int threads) {
+        return (int)std::max<size_t>(1, std::min<size_t>((226 * 1024) / (smem + 1024), 512 / threads));
+    }
+    static constexpr int KMINB = fit(KSMEM, KTHREADS), SMINB = fit(SSMEM, STHREADS), HMINB = fit(HSMEM, KTHREADS);
+};
+
 template <typename T, int DIR> struct FastStridedTma {
     template <int N> struct K {
         static int run(const Plan3& p, Specs<cplx_t<T>> sp, int nb, Strided s, int axis, const char* name,
                        double bytes, cudaStream_t st) {
+            constexpr bool duo = sizeof(T) == 4 && DuoCfg<N>::OK;
             typedef StridedTmaCfg<T, N> cfg;
-            typedef fast::TileShape<T, N, cfg::B> TS;
+            constexpr int B = duo ? 2 * DuoCfg<N>::SBP : cfg::B;
+            constexpr int THREADS = duo ? DuoCfg<N>::STHREADS : cfg::THREADS;
+            constexpr size_t SMEM = duo ? DuoCfg<N>::SSMEM : cfg::SMEM;
+            typedef fast::TileShape<T, N, B> TS;
             tma::Maps maps;
             for (int i = 0; i < nb; i++)
-                if (!spectrum_map(&maps.m[i], sp.p[i], p, sizeof(cplx_t<T>), cfg::B, axis == 1 ? TS::BOXL : 1,
+                if (!spectrum_map(&maps.m[i], sp.p[i], p, sizeof(cplx_t<T>), B, axis == 1 ? TS::BOXL : 1,
                                   axis == 1 ? 1 : TS::BOXL))
                     return TMA_UNAVAILABLE;
-            auto kern = fast::strided_tma<T, N, cfg::B, cfg::S, DIR>;
-            cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg::SMEM);
-            const int64_t ntiles = (int64_t)s.outer * ((s.ncols + cfg::B - 1) / cfg::B) * nb;
-            PRC_LAUNCH_B(name, st, bytes,
-                         kern<<<resident_grid(kern, cfg::THREADS, cfg::SMEM, ntiles), cfg::THREADS, cfg::SMEM, st>>>(
-                             maps, sp, nb, s, axis));
-            PRC_CHECK_LAUNCH();
-            return PRC_OK;
+            const int64_t ntiles = (int64_t)s.outer * ((s.ncols + B - 1) / B) * nb;
+            auto launch = [&](auto kern) {
+                cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM);
+                PRC_LAUNCH_B(name, st, bytes,
+                             kern<<<resident_grid(kern, THREADS, SMEM, ntiles), THREADS, SMEM, st>>>(maps, sp, nb, s, axis));
+                PRC_CHECK_LAUNCH();
+                return PRC_OK;
+            };
+            if constexpr (duo) return launch(fast::strided_duo<N, DuoCfg<N>::SBP, DuoCfg<N>::S, DIR, DuoCfg<N>::SMINB>);
+            else return launch(fast::strided_tma<T, N, cfg::B, cfg::S, DIR>);
         }
     };
 };
@@ -1067,34 +1097,41 @@ template <typename T, int N> struct KSpaceTmaCfg {
 template <typename T> struct FastXTma {
     template <int N> struct K {
         template <int KT>
-        static int go(const tma::Maps& maps, int nin, Specs<cplx_t<T>> so, const Plan3& p, KOp op, double bytes,
+        static int go(Specs<cplx_t<T>> si, int nin, Specs<cplx_t<T>> so, const Plan3& p, KOp op, double bytes,
                       cudaStream_t st) {
-            typedef KSpaceTmaCfg<T, N> cfg;
-            auto kern = fast::x_kspace_tma<T, N, cfg::B, cfg::S, KT, cfg::LEAN>;
-            cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg::SMEM);
-            const int64_t ntiles = (int64_t)p.dims.n[1] * ((p.nh + cfg::B - 1) / cfg::B) * nin;
-            PRC_LAUNCH_B("fft_x_kspace", st, bytes,
-                         kern<<<resident_grid(kern, cfg::THREADS, cfg::SMEM, ntiles), cfg::THREADS, cfg::SMEM, st>>>(
-                             maps, nin, so, p.dims, p.pitch, op));
-            PRC_CHECK_LAUNCH();
-            return PRC_OK;
+            constexpr bool duo = sizeof(T) == 4 && DuoCfg<N>::K_OK && (KT == KOP_GAUSS || KT == KOP_PP || KT == KOP_PSI || KT == KOP_HESS3);
+            constexpr int B = duo ? 2 * DuoCfg<N>::KBP : KSpaceTmaCfg<T, N>::B;
+            constexpr int THREADS = duo ? DuoCfg<N>::KTHREADS : KSpaceTmaCfg<T, N>::THREADS;
+            constexpr size_t SMEM = duo ? DuoCfg<N>::KSMEM : KSpaceTmaCfg<T, N>::SMEM;
+            typedef fast::TileShape<T, N, B> TS;
+            tma::Maps maps;
+            for (int i = 0; i < nin; i++)
+                if (!spectrum_map(&maps.m[i], si.p[i], p, sizeof(cplx_t<T>), B, 1, TS::BOXL)) return TMA_UNAVAILABLE;
+            if (duo)         // pairs of columns are stored as 16-byte vectors
+                for (int i = 0; i < nin * op.nper; i++)
+                    if (((uintptr_t)so.p[i] & 15) != 0) return TMA_UNAVAILABLE;
+            const int64_t ntiles = (int64_t)p.dims.n[1] * ((p.nh + B - 1) / B) * nin;
+            auto launch = [&](auto kern) {
+                cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM);
+                PRC_LAUNCH_B("fft_x_kspace", st, bytes,
+                             kern<<<resident_grid(kern, THREADS, SMEM, ntiles), THREADS, SMEM, st>>>(maps, nin, so, p.dims,
+                                                                                                  p.pitch, op));
+                PRC_CHECK_LAUNCH();
+                return PRC_OK;
+            };
+            if constexpr (duo) return launch(fast::x_kspace_duo<N, DuoCfg<N>::KBP, KT, DuoCfg<N>::KMINB>);
+            else return launch(fast::x_kspace_tma<T, N, B, KSpaceTmaCfg<T, N>::S, KT, KSpaceTmaCfg<T, N>::LEAN>);
         }
         static int run(const Plan3& p, Specs<cplx_t<T>> si, int nin, Specs<cplx_t<T>> so, KOp op, double bytes,
                        cudaStream_t st) {
-            typedef KSpaceTmaCfg<T, N> cfg;
-            typedef fast::TileShape<T, N, cfg::B> TS;
-            tma::Maps maps;
-            for (int i = 0; i < nin; i++)
-                if (!spectrum_map(&maps.m[i], si.p[i], p, sizeof(cplx_t<T>), cfg::B, 1, TS::BOXL))
-                    return TMA_UNAVAILABLE;
             switch (op.type) {
-                case KOP_GAUSS: return go<KOP_GAUSS>(maps, nin, so, p, op, bytes, st);
-                case KOP_PP: return go<KOP_PP>(maps, nin, so, p, op, bytes, st);
-                case KOP_ITER_GLOBAL: return go<KOP_ITER_GLOBAL>(maps, nin, so, p, op, bytes, st);
-                case KOP_ITER_LOCAL: return go<KOP_ITER_LOCAL>(maps, nin, so, p, op, bytes, st);
-                case KOP_PSI: return go<KOP_PSI>(maps, nin, so, p, op, bytes, st);
-                case KOP_HESS3: return go<KOP_HESS3>(maps, nin, so, p, op, bytes, st);
-                default: return go<KOP_IDENTITY>(maps, nin, so, p, op, bytes, st);
+                case KOP_GAUSS: return go<KOP_GAUSS>(si, nin, so, p, op, bytes, st);
+                case KOP_PP: return go<KOP_PP>(si, nin, so, p, op, bytes, st);
+                case KOP_ITER_GLOBAL: return go<KOP_ITER_GLOBAL>(si, nin, so, p, op, bytes, st);
+                case KOP_ITER_LOCAL: return go<KOP_ITER_LOCAL>(si, nin, so, p, op, bytes, st);
+                case KOP_PSI: return go<KOP_PSI>(si, nin, so, p, op, bytes, st);
+                case KOP_HESS3: return go<KOP_HESS3>(si, nin, so, p, op, bytes, st);
+                default: return go<KOP_IDENTITY>(si, nin, so, p, op, bytes, st);
             }
         }
     };
@@ -1140,10 +1177,14 @@ template <typename T> struct FastHessTma {
         // probe: only check that the tensor maps can be made (nothing is launched)
         static int run(const Plan3& p, cplx_t<T>* const* d, cplx_t<T>* const* o, fast::HessGeom h, cudaStream_t st,
                        bool probe) {
-            typedef fast::TileShape<T, N, cfg::B> TS;
+            constexpr bool use_duo = sizeof(T) == 4 && DuoCfg<N>::OK;
+            constexpr int B = use_duo ? 2 * DuoCfg<N>::KBP : cfg::B;
+            typedef fast::TileShape<T, N, B> TS;
             tma::Maps maps;
             for (int i = 0; i < 3; i++)
-                if (!spectrum_map(&maps.m[i], d[i], p, sizeof(cplx_t<T>), cfg::B, TS::BOXL, 1)) return TMA_UNAVAILABLE;
+                if (!spectrum_map(&maps.m[i], d[i], p, sizeof(cplx_t<T>), B, TS::BOXL, 1) ||
+                    (use_duo && ((uintptr_t)o[i] & 15) != 0))
+                    return TMA_UNAVAILABLE;
             if (probe) return PRC_OK;
             Specs<cplx_t<T>> so;
             for (int i = 0; i < 3; i++) so.p[i] = o[i];
@@ -1153,16 +1194,27 @@ template <typename T> struct FastHessTma {
             s.outer = p.dims.n[0];
             s.os = (int64_t)p.dims.n[1] * p.pitch;
             s.ncols = p.nh;
+            const int64_t ntiles = (int64_t)s.outer * ((s.ncols + B - 1) / B);
+            const double bytes = 6.0 * spectrum_values(p) * sizeof(cplx_t<T>);
+            if constexpr (use_duo) {
+                typedef DuoCfg<N> duo;
+                auto kern = fast::y_hessian_duo<N, duo::KBP, duo::S, duo::HMINB>;
+                cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)duo::HSMEM);
+                PRC_LAUNCH_B("fft_y_inv_hessian", st, bytes,
+                             kern<<<resident_grid(kern, duo::KTHREADS, duo::HSMEM, ntiles), duo::KTHREADS, duo::HSMEM, st>>>(
+                                 maps, so, s, h));
+                PRC_CHECK_LAUNCH();
+                return PRC_OK;
+            } else {
             auto kern = fast::y_hessian_tma<T, N, cfg::B, cfg::S, cfg::MINB, cfg::PP>;
             const size_t smem = cfg::SMEM + 2 * N * sizeof(T);     // + the x1 and k_y tables
             cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            const int64_t ntiles = (int64_t)s.outer * ((s.ncols + cfg::B - 1) / cfg::B);
-            const double bytes = 6.0 * spectrum_values(p) * sizeof(cplx_t<T>);
             PRC_LAUNCH_B("fft_y_inv_hessian", st, bytes,
                          kern<<<resident_grid(kern, cfg::THREADS, smem, ntiles), cfg::THREADS, smem, st>>>(
                              maps, so, s, h));
             PRC_CHECK_LAUNCH();
             return PRC_OK;
+            }
         }
     };
 };
