@@ -157,22 +157,38 @@ __device__ __forceinline__ void dft_generic(C* v, const C* __restrict__ tw, int 
     for (int m = 0; m < R; m++) v[m] = out[m];
 }
 
-// One Stockham pass of radix R over B lines of length n stored (k, line) at k * bp + line.
+// Quotients by a number that a launch or a pass fixes: one multiplication.  Exact for q d < 2^32 (here q < 2^16 values of
+// a tile, d at most 2048).
+struct FastDiv {
+    uint32_t d, m;
+    __device__ __forceinline__ explicit FastDiv(int d_) : d(d_), m(d_ > 1 ? 0xffffffffu / (uint32_t)d_ + 1u : 0u) {}
+    __device__ __forceinline__ int div(int q) const { return d > 1 ? (int)__umulhi((uint32_t)q, m) : q; }
+    __device__ __forceinline__ int mod(int q, int quotient) const { return q - quotient * (int)d; }
+};
+
+// log2 of a tile's lines (a power of two).
+__device__ __forceinline__ int log2_of(int B) { return 31 - __clz(B); }
+
+// One Stockham pass of radix R over B (a power of two) lines of length n stored (k, line) at k * bp + line.  The passes
+// of these kernels were bound by integer divisions, one for each of line, j mod Ns and every twiddle's exponent.  Shifts,
+// FastDiv and exponents that stay below n (r k < R Ns), with all the blocks that fit on an SM instead of two, took the
+// transforms of a 150 x 125 x 243 reconstruction (FP32, 25 passes) from 2.62 to 1.73 ms.
 template <typename C, int DIR, int R>
 __device__ __forceinline__ void stockham_pass(const C* __restrict__ src, C* __restrict__ dst, int n, int B, int bp,
                                               int Ns, const C* __restrict__ tw, int tws) {
-    const int nb = n / R;
-    const int twstep = n / (Ns * R);
+    const int nb = n / R, lb = log2_of(B);
+    const int twstep = n / (Ns * R) * tws;
+    const FastDiv by_ns(Ns);
     for (int q = threadIdx.x; q < nb * B; q += blockDim.x) {
-        const int line = q % B, j = q / B;
-        const int k = j % Ns;
+        const int line = q & (B - 1), j = q >> lb;
+        const int k = by_ns.mod(j, by_ns.div(j));
         C v[R];
 #pragma unroll
         for (int r = 0; r < R; r++) v[r] = src[(j + r * nb) * bp + line];
         if (k > 0) {
 #pragma unroll
             for (int r = 1; r < R; r++) {
-                C w = tw[((r * k * twstep) % n) * tws];
+                C w = tw[r * k * twstep];
                 if (DIR > 0) w = cconj(w);
                 v[r] = cmul(v[r], w);
             }
@@ -196,13 +212,14 @@ __device__ __forceinline__ void stockham_pass(const C* __restrict__ src, C* __re
 template <typename C, int DIR>
 __device__ __forceinline__ void stockham_pass_any(const C* __restrict__ src, C* __restrict__ dst, int n, int B, int bp,
                                                   int Ns, int R, const C* __restrict__ tw, int tws) {
-    const int nb = n / R;
+    const int nb = n / R, lb = log2_of(B);
     const int twstep = n / (Ns * R);
+    const FastDiv by_ns(Ns), by_nb(nb);
     for (int q = threadIdx.x; q < n * B; q += blockDim.x) {
-        const int line = q % B, rest = q / B;
-        const int j = rest % nb, m = rest / nb;
-        const int k = j % Ns;
-        const int E = (k * twstep + m * nb) % n;
+        const int line = q & (B - 1), rest = q >> lb;
+        const int m = by_nb.div(rest), j = by_nb.mod(rest, m);
+        const int k = by_ns.mod(j, by_ns.div(j));
+        const int E = k * twstep + m * nb;         // below n: k twstep < nb
         C acc = src[j * bp + line];
         int ex = 0;
         for (int r = 1; r < R; r++) {
@@ -273,7 +290,8 @@ __global__ void __launch_bounds__(FFT_THREADS) fft_z_r2c(RealsIn in, Specs<cplx_
     const bool full = (n2 & 1) != 0;
     const int M = full ? n2 : n2 / 2;              // transform length
     const int L = full ? n2 : M + 1;               // buffer rows
-    const int bp = row_pitch(B);
+    const int bp = row_pitch(B), lb = log2_of(B);
+    const FastDiv by_n2(n2), by_nh(nh), by_m(M);
     C* tw = (C*)smem_raw;                          // n2 entries
     C* bufa = tw + n2;                             // L * bp
     C* bufb = bufa + L * bp;
@@ -289,13 +307,13 @@ __global__ void __launch_bounds__(FFT_THREADS) fft_z_r2c(RealsIn in, Specs<cplx_
         const TIN* src = (const TIN*)in.p[bi] + row0 * n2;
         if (full) {
             for (int q = threadIdx.x; q < B * n2; q += blockDim.x) {
-                const int line = q / n2, m = q % n2;
+                const int line = by_n2.div(q), m = by_n2.mod(q, line);
                 bufa[m * bp + line] = cmake<C>(line < nrow ? (T)src[(int64_t)line * n2 + m] : (T)0, (T)0);
             }
         } else {
             // load rows as complex pairs (x[2m], x[2m+1])
             for (int q = threadIdx.x; q < B * M; q += blockDim.x) {
-                const int line = q / M, m = q % M;
+                const int line = by_m.div(q), m = by_m.mod(q, line);
                 C v = cmake<C>((T)0, (T)0);
                 if (line < nrow) {
                     const TIN* r = src + (int64_t)line * n2 + 2 * m;
@@ -311,7 +329,7 @@ __global__ void __launch_bounds__(FFT_THREADS) fft_z_r2c(RealsIn in, Specs<cplx_
             x = z == bufa ? bufb : bufa;
             // unpack: X[k] = (Z[k] + conj Z[M-k]) / 2 - i w^k (Z[k] - conj Z[M-k]) / 2
             for (int q = threadIdx.x; q < B * nh; q += blockDim.x) {
-                const int line = q % B, k = q / B;
+                const int line = q & (B - 1), k = q >> lb;
                 const C zk = z[(k == M ? 0 : k) * bp + line];
                 const C zc = cconj(z[(k == 0 ? 0 : M - k) * bp + line]);
                 const C e = cscale(cadd(zk, zc), (T)0.5);
@@ -322,7 +340,7 @@ __global__ void __launch_bounds__(FFT_THREADS) fft_z_r2c(RealsIn in, Specs<cplx_
         }
         C* dst = out.p[bi] + row0 * pitch;
         for (int q = threadIdx.x; q < B * nh; q += blockDim.x) {
-            const int line = q / nh, k = q % nh;
+            const int line = by_nh.div(q), k = by_nh.mod(q, line);
             if (line < nrow) dst[(int64_t)line * pitch + k] = x[k * bp + line];
         }
         __syncthreads();
@@ -343,16 +361,18 @@ struct Strided {
 
 template <typename C>
 __device__ __forceinline__ void load_tile(C* buf, const C* __restrict__ g, const Strided& s, int B, int cols) {
+    const int lb = log2_of(B);
     for (int q = threadIdx.x; q < s.n * B; q += blockDim.x) {
-        const int k = q / B, col = q % B;
+        const int k = q >> lb, col = q & (B - 1);
         buf[k * B + col] = col < cols ? g[(int64_t)k * s.ls + col] : cmake<C>(0, 0);
     }
 }
 
 template <typename C>
 __device__ __forceinline__ void store_tile(C* __restrict__ g, const C* buf, const Strided& s, int B, int cols) {
+    const int lb = log2_of(B);
     for (int q = threadIdx.x; q < s.n * B; q += blockDim.x) {
-        const int k = q / B, col = q % B;
+        const int k = q >> lb, col = q & (B - 1);
         if (col < cols) g[(int64_t)k * s.ls + col] = buf[k * B + col];
     }
 }
@@ -487,7 +507,7 @@ __global__ void __launch_bounds__(FFT_THREADS) fft_x_fused(Specs<cplx_t<T>> in, 
     s.outer = n1;
     s.os = pitch;
     s.ncols = nh;
-    const int ctiles = (nh + B - 1) / B;
+    const int ctiles = (nh + B - 1) / B, lb = log2_of(B);
     const int64_t tiles_per = (int64_t)n1 * ctiles;
     const int64_t ntiles = tiles_per * nin;
     for (int64_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
@@ -504,7 +524,7 @@ __global__ void __launch_bounds__(FFT_THREADS) fft_x_fused(Specs<cplx_t<T>> in, 
         __syncthreads();
         for (int o = 0; o < op.nper; o++) {
             for (int q = threadIdx.x; q < n0 * B; q += blockDim.x) {
-                const int ix = q / B, col = q % B;
+                const int ix = q >> lb, col = q & (B - 1);
                 const double2 m = kmultiplier(op, o, ix, iy, c0 + col);
                 const C v = spec[q];
                 bufa[q] = cmake<C>((T)(m.x * (double)v.x - m.y * (double)v.y), (T)(m.x * (double)v.y + m.y * (double)v.x));
@@ -563,7 +583,7 @@ __device__ __forceinline__ T epilogue_value(const Epi<T>& e, const T* vals, int 
             break;
         }
         case EPI_ITER_LOCAL: {
-            const int ix = (int)(row / dims.n[1]), iy = (int)(row % dims.n[1]);
+            const int ix = (int)((uint32_t)row / (uint32_t)dims.n[1]), iy = (int)(row - (int64_t)ix * dims.n[1]);
             const double x[3] = {e.offset[0] + e.cell[0] * ix, e.offset[1] + e.cell[1] * iy,
                                  e.offset[2] + e.cell[2] * iz};
             const double x2 = (x[0] * x[0] + x[1] * x[1]) + x[2] * x[2];
@@ -577,7 +597,7 @@ __device__ __forceinline__ T epilogue_value(const Epi<T>& e, const T* vals, int 
         case EPI_ITER_POLY: {
             // inputs C, B, A of the quadratic in x2 formed by the Hessian y pass: the RSD term is
             // ((C x2 + B) x2 + A) / |x|^2
-            const int ix = (int)(row / dims.n[1]), iy = (int)(row % dims.n[1]);
+            const int ix = (int)((uint32_t)row / (uint32_t)dims.n[1]), iy = (int)(row - (int64_t)ix * dims.n[1]);
             const double x0 = e.offset[0] + e.cell[0] * ix, x1 = e.offset[1] + e.cell[1] * iy;
             const double xz = e.offset[2] + e.cell[2] * iz;
             const double x2 = (x0 * x0 + x1 * x1) + xz * xz;
@@ -621,7 +641,8 @@ __global__ void __launch_bounds__(FFT_THREADS) fft_z_c2r(Specs<cplx_t<T>> in, in
     const bool full = (n2 & 1) != 0;
     const int M = full ? n2 : n2 / 2;          // transform length
     const int L = full ? n2 : nh;              // buffer rows
-    const int bp = row_pitch(B);
+    const int bp = row_pitch(B), lb = log2_of(B);
+    const FastDiv by_n2(n2), by_nh(nh), by_m(M);
     C* tw = (C*)smem_raw;                    // n2
     C* bufa = tw + n2;                       // L * bp
     C* bufb = bufa + L * bp;                 // L * bp
@@ -636,26 +657,26 @@ __global__ void __launch_bounds__(FFT_THREADS) fft_z_c2r(Specs<cplx_t<T>> in, in
         for (int i = 0; i < nin; i++) {
             const C* src = in.p[i] + row0 * pitch;
             for (int q = threadIdx.x; q < B * nh; q += blockDim.x) {
-                const int line = q / nh, k = q % nh;
+                const int line = by_nh.div(q), k = by_nh.mod(q, line);
                 bufa[k * bp + line] = line < nrow ? src[(int64_t)line * pitch + k] : cmake<C>(0, 0);
             }
             __syncthreads();
             C* z;
             if (full) {
                 for (int q = threadIdx.x; q < B * (n2 - nh); q += blockDim.x) {
-                    const int line = q % B, k = nh + q / B;
+                    const int line = q & (B - 1), k = nh + (q >> lb);
                     bufa[k * bp + line] = cconj(bufa[(n2 - k) * bp + line]);
                 }
                 __syncthreads();
                 z = fft_lines<C, +1>(bufa, bufb, n2, B, bp, rd, tw, 1);
                 for (int q = threadIdx.x; q < B * n2; q += blockDim.x) {
-                    const int line = q / n2, m = q % n2;
+                    const int line = by_n2.div(q), m = by_n2.mod(q, line);
                     acc[((int64_t)i * B + line) * n2 + m] = (T)(z[m * bp + line].x * e.scale);
                 }
             } else {
                 // pack: Z[k] = (X[k] + conj X[M-k]) + i w^-k (X[k] - conj X[M-k]), k < M
                 for (int q = threadIdx.x; q < B * M; q += blockDim.x) {
-                    const int line = q % B, k = q / B;
+                    const int line = q & (B - 1), k = q >> lb;
                     const C xk = bufa[k * bp + line];
                     const C xc = cconj(bufa[(M - k) * bp + line]);
                     const C ev = cadd(xk, xc);
@@ -666,7 +687,7 @@ __global__ void __launch_bounds__(FFT_THREADS) fft_z_c2r(Specs<cplx_t<T>> in, in
                 z = fft_lines<C, +1>(bufb, bufa, M, B, bp, rd, tw, 2);
                 // (x[2m], x[2m+1]) * scale
                 for (int q = threadIdx.x; q < B * M; q += blockDim.x) {
-                    const int line = q / M, m = q % M;
+                    const int line = by_m.div(q), m = by_m.mod(q, line);
                     const C v = z[m * bp + line];
                     T* a = acc + ((int64_t)i * B + line) * n2 + 2 * m;
                     a[0] = (T)(v.x * e.scale);
@@ -676,7 +697,7 @@ __global__ void __launch_bounds__(FFT_THREADS) fft_z_c2r(Specs<cplx_t<T>> in, in
             __syncthreads();
         }
         for (int q = threadIdx.x; q < B * n2; q += blockDim.x) {
-            const int line = q / n2, iz = q % n2;
+            const int line = by_n2.div(q), iz = by_n2.mod(q, line);
             if (line >= nrow) continue;
             epilogue_store(e, nin, acc + (int64_t)line * n2 + iz, B * n2, row0 + line, iz, dims);
         }
@@ -749,16 +770,15 @@ template <typename T> static void pad_pitch(Plan3* p) {
     p->pitch = (p->nh + q - 1) / q * q;
 }
 
-// Lines per tile B (power of two) so that `nbuf` buffers of n * B complex fit the budget.
-static int choose_B(int n, int nbuf, size_t csize, size_t budget, int bmax) {
-    int B = bmax;
-    while (B > 1 && (size_t)nbuf * n * B * csize > budget) B >>= 1;
+// Lines per tile B (a power of two) of a mixed-radix kernel whose blocks of B lines need `need(B)` bytes of shared memory:
+// 16, or 8 where three blocks of 16 do not fit on an SM, fewer still while two do not.  Plane-parallel passes of 500 x 450 x
+// 300 in FP32: 5.55 ms, 6.84 with 16 lines wherever two blocks fit; 360^3 3.83 and 4.08; 250^3 in FP64 2.13 and 2.11; 8
+// lines already where four blocks do not fit cost 150 x 125 x 243 a hundredth.
+template <typename Need> static int choose_B(const Need& need) {
+    int B = 16;
+    while (B > 8 && need(B) > (size_t)60 * 1024) B >>= 1;
+    while (B > 1 && need(B) > (size_t)100 * 1024) B >>= 1;
     return B;
-}
-
-static int fft_grid(int64_t ntiles, int ctas_per_sm) {
-    int64_t cap = (int64_t)device_sm_count() * ctas_per_sm;
-    return (int)std::max<int64_t>(1, std::min<int64_t>(ntiles, cap));
 }
 
 // Lengths of the register-resident kernels: powers of two from 8 to MAX_FAST_N, and 96, 192, 384 (three
@@ -1258,7 +1278,6 @@ template <typename T> struct FastZC2RTma {
 template <typename T> struct FFTLaunch {
     typedef cplx_t<T> C;
     static constexpr size_t CS = sizeof(C);
-    static constexpr size_t BUDGET = 100 * 1024;
 
     template <typename TIN>
     static int z_r2c(const Plan3& p, const void* const* in, C* const* out, int nb, cudaStream_t st) {
@@ -1275,8 +1294,7 @@ template <typename T> struct FFTLaunch {
         }
         const int n2 = p.dims.n[2], L = n2 % 2 ? n2 : n2 / 2 + 1;
         auto need = [&](int b) { return (size_t)(2 * L * row_pitch(b) + n2) * CS; };
-        int B = 16;
-        while (B > 1 && need(B) > BUDGET) B >>= 1;
+        const int B = choose_B(need);
         const size_t smem = need(B);
         RealsIn ri;
         Specs<C> so;
@@ -1287,7 +1305,7 @@ template <typename T> struct FFTLaunch {
         cudaFuncSetAttribute(fft_z_r2c<T, TIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         int64_t rows = (int64_t)p.dims.n[0] * p.dims.n[1];
         int64_t ntiles = ((rows + B - 1) / B) * nb;
-        PRC_LAUNCH_B("fft_z_r2c", st, (double)nb * rows * (p.dims.n[2] * sizeof(TIN) + p.nh * CS), fft_z_r2c<T, TIN><<<fft_grid(ntiles, 2), FFT_THREADS, smem, st>>>(ri, so, nb, p.dims, p.pitch, p.rz, B));
+        PRC_LAUNCH_B("fft_z_r2c", st, (double)nb * rows * (p.dims.n[2] * sizeof(TIN) + p.nh * CS), fft_z_r2c<T, TIN><<<resident_grid(fft_z_r2c<T, TIN>, FFT_THREADS, smem, ntiles), FFT_THREADS, smem, st>>>(ri, so, nb, p.dims, p.pitch, p.rz, B));
         PRC_CHECK_LAUNCH();
         return PRC_OK;
     }
@@ -1333,13 +1351,14 @@ template <typename T> struct FFTLaunch {
             s.os = p.pitch;
         }
         s.ncols = nh;
-        int B = choose_B(s.n, 2, CS, BUDGET - s.n * CS, 16);
-        size_t smem = (size_t)(2 * s.n * B + s.n) * CS;
+        auto need = [&](int b) { return (size_t)(2 * s.n * b + s.n) * CS; };
+        const int B = choose_B(need);
+        const size_t smem = need(B);
         Specs<C> sp;
         for (int i = 0; i < nb; i++) sp.p[i] = data[i];
         cudaFuncSetAttribute(fft_strided<T, DIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         int64_t ntiles = (int64_t)s.outer * ((nh + B - 1) / B) * nb;
-        PRC_LAUNCH_B((DIR < 0 ? (axis == 1 ? "fft_y_fwd" : "fft_x_fwd") : (axis == 1 ? "fft_y_inv" : "fft_x_inv")), st, 2.0 * nb * spectrum_values(p) * CS, fft_strided<T, DIR><<<fft_grid(ntiles, 2), FFT_THREADS, smem, st>>>(sp, nb, s, axis == 1 ? p.ry : p.rx, B));
+        PRC_LAUNCH_B((DIR < 0 ? (axis == 1 ? "fft_y_fwd" : "fft_x_fwd") : (axis == 1 ? "fft_y_inv" : "fft_x_inv")), st, 2.0 * nb * spectrum_values(p) * CS, fft_strided<T, DIR><<<resident_grid(fft_strided<T, DIR>, FFT_THREADS, smem, ntiles), FFT_THREADS, smem, st>>>(sp, nb, s, axis == 1 ? p.ry : p.rx, B));
         PRC_CHECK_LAUNCH();
         return PRC_OK;
     }
@@ -1357,14 +1376,15 @@ template <typename T> struct FFTLaunch {
             }
             return dispatch_pow2<FastX<T>::template K>(n0, si, nin, so, p.dims, p.pitch, op, bytes, st);
         }
-        int B = choose_B(n0, 3, CS, BUDGET - n0 * CS, 16);
-        size_t smem = (size_t)(3 * n0 * B + n0) * CS;
+        auto need = [&](int b) { return (size_t)(3 * n0 * b + n0) * CS; };
+        const int B = choose_B(need);
+        const size_t smem = need(B);
         Specs<C> si, so;
         for (int i = 0; i < nin; i++) si.p[i] = in[i];
         for (int i = 0; i < nin * op.nper; i++) so.p[i] = out[i];
         cudaFuncSetAttribute(fft_x_fused<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         int64_t ntiles = (int64_t)p.dims.n[1] * ((p.nh + B - 1) / B) * nin;
-        PRC_LAUNCH_B("fft_x_kspace", st, (double)nin * (1 + op.nper) * spectrum_values(p) * CS, fft_x_fused<T><<<fft_grid(ntiles, 2), FFT_THREADS, smem, st>>>(si, nin, so, p.dims, p.pitch, p.rx, B, op));
+        PRC_LAUNCH_B("fft_x_kspace", st, (double)nin * (1 + op.nper) * spectrum_values(p) * CS, fft_x_fused<T><<<resident_grid(fft_x_fused<T>, FFT_THREADS, smem, ntiles), FFT_THREADS, smem, st>>>(si, nin, so, p.dims, p.pitch, p.rx, B, op));
         PRC_CHECK_LAUNCH();
         return PRC_OK;
     }
@@ -1402,15 +1422,14 @@ template <typename T> struct FFTLaunch {
         auto need = [&](int b) {
             return (size_t)(2 * L * row_pitch(b) + n2) * CS + (size_t)nin * b * n2 * sizeof(T);
         };
-        int B = 16;
-        while (B > 1 && need(B) > BUDGET) B >>= 1;
+        const int B = choose_B(need);
         const size_t smem = need(B);
         Specs<C> si;
         for (int i = 0; i < nin; i++) si.p[i] = in[i];
         cudaFuncSetAttribute(fft_z_c2r<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         int64_t rows = (int64_t)p.dims.n[0] * p.dims.n[1];
         int64_t ntiles = (rows + B - 1) / B;
-        PRC_LAUNCH_B("fft_z_c2r", st, (double)nin * rows * nh * CS + (double)rows * p.dims.n[2] * sizeof(T) * (e.type == EPI_STORE ? nin : (e.delta ? 2 : 1)), fft_z_c2r<T><<<fft_grid(ntiles, 2), FFT_THREADS, smem, st>>>(si, nin, p.dims, p.pitch, p.rz, B, e));
+        PRC_LAUNCH_B("fft_z_c2r", st, (double)nin * rows * nh * CS + (double)rows * p.dims.n[2] * sizeof(T) * (e.type == EPI_STORE ? nin : (e.delta ? 2 : 1)), fft_z_c2r<T><<<resident_grid(fft_z_c2r<T>, FFT_THREADS, smem, ntiles), FFT_THREADS, smem, st>>>(si, nin, p.dims, p.pitch, p.rz, B, e));
         PRC_CHECK_LAUNCH();
         return PRC_OK;
     }
