@@ -13,6 +13,7 @@ host-to-device copies asynchronous) or CUDA tensors; results come back in the sa
 container.  ``dtype='f4'`` runs the FP32 pipeline with FP64 cloud-in-cell sums, FP64
 normalisation and (multigrid) FP64 defect correction; ``dtype='f8'`` runs everything in FP64.
 """
+import logging
 import weakref
 
 import numpy as np
@@ -84,7 +85,8 @@ class BaseReconstruction(BaseClass):
         with self._stream_ctx():
             self.mesh_data = self._new_paint_mesh()
             self.mesh_randoms = self._new_paint_mesh()
-        self.log_info('Using mesh {}.'.format(self.mesh_data))
+        if self.logger.isEnabledFor(logging.INFO):      # the mesh's numpy vectors take 0.1 ms to print
+            self.log_info('Using mesh {}.'.format(self.mesh_data))
         del torch
 
     def _stream_ctx(self):
