@@ -730,7 +730,7 @@ __global__ void __launch_bounds__(PULL_WARPS * 32) paint_pull(const uint32_t* __
         return;
     }
     for (int64_t c = (int64_t)blockIdx.x * PULL_WARPS + warp; c < ncol; c += (int64_t)gridDim.x * PULL_WARPS) {
-        const int X = (int)(c / n1), Y = (int)(c % n1);
+        const int X = (int)((uint32_t)c / (uint32_t)n1), Y = (int)((uint32_t)c - (uint32_t)X * (uint32_t)n1);
         for (int z = lane; z < n2; z += 32) col[z] = 0.;
         __syncwarp();
         // base columns contributing corner (cx, cy) to this column, in a fixed order
@@ -746,7 +746,7 @@ __global__ void __launch_bounds__(PULL_WARPS * 32) paint_pull(const uint32_t* __
                 int iz = INT_MAX;
                 double a = 0., b = 0.;
                 if (ok) {
-                    iz = (int)(keys[i] % (uint32_t)n2);
+                    iz = (int)(keys[i] - (uint32_t)src * (uint32_t)n2);     // keys of column src: src n2 + iz
                     const Payload<F> pl = payload[i];
                     const F wx = cx ? pl.t[0] : rn_sub((F)1, pl.t[0]);
                     const F wy = cy ? pl.t[1] : rn_sub((F)1, pl.t[1]);
