@@ -172,10 +172,11 @@ __device__ __forceinline__ int log2_of(int B) { return 31 - __clz(B); }
 // One Stockham pass of radix R over B (a power of two) lines of length n stored (k, line) at k * bp + line.  The passes
 // of these kernels were bound by integer divisions, one for each of line, j mod Ns and every twiddle's exponent.  Shifts,
 // FastDiv and exponents that stay below n (r k < R Ns), with all the blocks that fit on an SM instead of two, took the
-// transforms of a 150 x 125 x 243 reconstruction (FP32, 25 passes) from 2.62 to 1.73 ms.
-template <typename C, int DIR, int R>
-__device__ __forceinline__ void stockham_pass(const C* __restrict__ src, C* __restrict__ dst, int n, int B, int bp,
-                                              int Ns, const C* __restrict__ tw, int tws) {
+// transforms of a 150 x 125 x 243 reconstruction (FP32, 25 passes) from 2.62 to 1.73 ms; strided tiles that the first pass
+// reads from global memory and the last one writes there (fft_lines_through) to 1.54.
+template <typename C, int DIR, int R, class Src, class Dst>
+__device__ __forceinline__ void stockham_pass(const Src& src, const Dst& dst, int n, int B, int Ns,
+                                              const C* __restrict__ tw, int tws) {
     const int nb = n / R, lb = log2_of(B);
     const int twstep = n / (Ns * R) * tws;
     const FastDiv by_ns(Ns);
@@ -184,7 +185,7 @@ __device__ __forceinline__ void stockham_pass(const C* __restrict__ src, C* __re
         const int k = by_ns.mod(j, by_ns.div(j));
         C v[R];
 #pragma unroll
-        for (int r = 0; r < R; r++) v[r] = src[(j + r * nb) * bp + line];
+        for (int r = 0; r < R; r++) v[r] = src(j + r * nb, line);
         if (k > 0) {
 #pragma unroll
             for (int r = 1; r < R; r++) {
@@ -201,7 +202,7 @@ __device__ __forceinline__ void stockham_pass(const C* __restrict__ src, C* __re
         else dft_generic<C, DIR, R>(v, tw, n, tws);
         const int d = (j - k) * R + k;
 #pragma unroll
-        for (int r = 0; r < R; r++) dst[(d + r * Ns) * bp + line] = v[r];
+        for (int r = 0; r < R; r++) dst(d + r * Ns, line, v[r]);
     }
 }
 
@@ -209,9 +210,9 @@ __device__ __forceinline__ void stockham_pass(const C* __restrict__ src, C* __re
 // m of one R-point sub-transform, y_m = sum_r x_r w_{Ns R}^{r k} w_R^{r m} = sum_r x_r w_n^{r E},
 // E = k twstep + m nb (input twiddle and DFT kernel in one table lookup, exponent kept mod n by
 // addition); O(R) operations per output.
-template <typename C, int DIR>
-__device__ __forceinline__ void stockham_pass_any(const C* __restrict__ src, C* __restrict__ dst, int n, int B, int bp,
-                                                  int Ns, int R, const C* __restrict__ tw, int tws) {
+template <typename C, int DIR, class Src, class Dst>
+__device__ __forceinline__ void stockham_pass_any(const Src& src, const Dst& dst, int n, int B, int Ns, int R,
+                                                  const C* __restrict__ tw, int tws) {
     const int nb = n / R, lb = log2_of(B);
     const int twstep = n / (Ns * R);
     const FastDiv by_ns(Ns), by_nb(nb);
@@ -220,40 +221,91 @@ __device__ __forceinline__ void stockham_pass_any(const C* __restrict__ src, C* 
         const int m = by_nb.div(rest), j = by_nb.mod(rest, m);
         const int k = by_ns.mod(j, by_ns.div(j));
         const int E = k * twstep + m * nb;         // below n: k twstep < nb
-        C acc = src[j * bp + line];
+        C acc = src(j, line);
         int ex = 0;
         for (int r = 1; r < R; r++) {
             ex += E;
             if (ex >= n) ex -= n;
             C w = tw[ex * tws];
             if (DIR > 0) w = cconj(w);
-            acc = cadd(acc, cmul(src[(j + r * nb) * bp + line], w));
+            acc = cadd(acc, cmul(src(j + r * nb, line), w));
         }
-        dst[((j - k) * R + k + m * Ns) * bp + line] = acc;
+        dst((j - k) * R + k + m * Ns, line, acc);
     }
 }
 
-// Transforms B lines in place-ish: data in `a`, scratch `b`; returns the buffer with the result.
-// tw holds w_{n*tws}^m (so entry m*tws is w_n^m).
-template <typename C, int DIR>
-__device__ C* fft_lines(C* a, C* b, int n, int B, int bp, const Radices& rd, const C* __restrict__ tw, int tws) {
-    int Ns = 1;
-    for (int p = 0; p < rd.count; p++) {
-        const int R = rd.r[p];
-        switch (R) {
-            case 8: stockham_pass<C, DIR, 8>(a, b, n, B, bp, Ns, tw, tws); break;
-            case 4: stockham_pass<C, DIR, 4>(a, b, n, B, bp, Ns, tw, tws); break;
-            case 2: stockham_pass<C, DIR, 2>(a, b, n, B, bp, Ns, tw, tws); break;
-            case 3: stockham_pass<C, DIR, 3>(a, b, n, B, bp, Ns, tw, tws); break;
-            case 5: stockham_pass<C, DIR, 5>(a, b, n, B, bp, Ns, tw, tws); break;
-            case 7: stockham_pass<C, DIR, 7>(a, b, n, B, bp, Ns, tw, tws); break;
-            default: stockham_pass_any<C, DIR>(a, b, n, B, bp, Ns, R, tw, tws); break;
-        }
+template <typename C, int DIR, class Src, class Dst>
+__device__ __forceinline__ void stockham_any(const Src& src, const Dst& dst, int n, int B, int Ns, int R,
+                                             const C* __restrict__ tw, int tws) {
+    switch (R) {
+        case 8: stockham_pass<C, DIR, 8>(src, dst, n, B, Ns, tw, tws); break;
+        case 4: stockham_pass<C, DIR, 4>(src, dst, n, B, Ns, tw, tws); break;
+        case 2: stockham_pass<C, DIR, 2>(src, dst, n, B, Ns, tw, tws); break;
+        case 3: stockham_pass<C, DIR, 3>(src, dst, n, B, Ns, tw, tws); break;
+        case 5: stockham_pass<C, DIR, 5>(src, dst, n, B, Ns, tw, tws); break;
+        case 7: stockham_pass<C, DIR, 7>(src, dst, n, B, Ns, tw, tws); break;
+        default: stockham_pass_any<C, DIR>(src, dst, n, B, Ns, R, tw, tws); break;
+    }
+}
+
+// Lines in shared memory, element k of a line at k * bp + line.
+template <typename C> struct LinesIn {
+    const C* p;
+    int bp;
+    __device__ __forceinline__ C operator()(int k, int line) const { return p[k * bp + line]; }
+};
+template <typename C> struct LinesOut {
+    C* p;
+    int bp;
+    __device__ __forceinline__ void operator()(int k, int line, C v) const { p[k * bp + line] = v; }
+};
+
+// Two of a strided tile's trips through shared memory and two barriers less than staging it: y passes of 150 x 125 x 243
+// 0.38 -> 0.28 ms a reconstruction, k-space pass 0.48 -> 0.40 (its multipliers stay a step of their own: within the first
+// pass's butterflies they took 0.41).  80 registers (FP32) keep three blocks on an SM.
+// Transforms B lines: the first pass takes its elements from `first`, the last one gives them to `last` (both may be global
+// memory, the same lines), the passes between go through the buffers a and b.  The caller synchronises before a and b are
+// used again.  tw holds w_{n*tws}^m (so entry m*tws is w_n^m).
+template <typename C, int DIR, class First, class Last>
+__device__ __forceinline__ void fft_lines_through(const First& first, const Last& last, C* a, C* b, int n, int B, int bp,
+                                                  const Radices& rd, const C* __restrict__ tw, int tws) {
+    const int lb = log2_of(B);
+    if (rd.r[0] > 8) {
+        // direct summation reads each element R times
+        for (int q = threadIdx.x; q < n * B; q += blockDim.x) b[(q >> lb) * bp + (q & (B - 1))] = first(q >> lb, q & (B - 1));
+        __syncthreads();
+        stockham_pass_any<C, DIR>(LinesIn<C>{b, bp}, LinesOut<C>{a, bp}, n, B, 1, rd.r[0], tw, tws);
+    } else {
+        stockham_any<C, DIR>(first, LinesOut<C>{a, bp}, n, B, 1, rd.r[0], tw, tws);
+    }
+    __syncthreads();
+    if (rd.count == 1) {
+        for (int q = threadIdx.x; q < n * B; q += blockDim.x) last(q >> lb, q & (B - 1), a[(q >> lb) * bp + (q & (B - 1))]);
+        return;
+    }
+    int Ns = rd.r[0];
+    for (int p = 1; p + 1 < rd.count; p++) {
+        stockham_any<C, DIR>(LinesIn<C>{a, bp}, LinesOut<C>{b, bp}, n, B, Ns, rd.r[p], tw, tws);
         __syncthreads();
         C* t = a;
         a = b;
         b = t;
-        Ns *= R;
+        Ns *= rd.r[p];
+    }
+    stockham_any<C, DIR>(LinesIn<C>{a, bp}, last, n, B, Ns, rd.r[rd.count - 1], tw, tws);
+}
+
+// Transforms B lines in place-ish: data in `a`, scratch `b`; returns the buffer with the result.
+template <typename C, int DIR>
+__device__ C* fft_lines(C* a, C* b, int n, int B, int bp, const Radices& rd, const C* __restrict__ tw, int tws) {
+    int Ns = 1;
+    for (int p = 0; p < rd.count; p++) {
+        stockham_any<C, DIR>(LinesIn<C>{a, bp}, LinesOut<C>{b, bp}, n, B, Ns, rd.r[p], tw, tws);
+        __syncthreads();
+        C* t = a;
+        a = b;
+        b = t;
+        Ns *= rd.r[p];
     }
     return a;
 }
@@ -359,26 +411,24 @@ struct Strided {
     int ncols;      // columns (z extent nh)
 };
 
-template <typename C>
-__device__ __forceinline__ void load_tile(C* buf, const C* __restrict__ g, const Strided& s, int B, int cols) {
-    const int lb = log2_of(B);
-    for (int q = threadIdx.x; q < s.n * B; q += blockDim.x) {
-        const int k = q >> lb, col = q & (B - 1);
-        buf[k * B + col] = col < cols ? g[(int64_t)k * s.ls + col] : cmake<C>(0, 0);
+// The first pass reads a tile and the last one writes it directly (B columns of a row are 64 to 256 contiguous bytes).
+template <typename C> struct TileIn {
+    const C* g;
+    int64_t ls;
+    int cols;
+    __device__ __forceinline__ C operator()(int k, int col) const { return col < cols ? g[k * ls + col] : cmake<C>(0, 0); }
+};
+template <typename C> struct TileOut {
+    C* g;
+    int64_t ls;
+    int cols;
+    __device__ __forceinline__ void operator()(int k, int col, C v) const {
+        if (col < cols) g[k * ls + col] = v;
     }
-}
-
-template <typename C>
-__device__ __forceinline__ void store_tile(C* __restrict__ g, const C* buf, const Strided& s, int B, int cols) {
-    const int lb = log2_of(B);
-    for (int q = threadIdx.x; q < s.n * B; q += blockDim.x) {
-        const int k = q >> lb, col = q & (B - 1);
-        if (col < cols) g[(int64_t)k * s.ls + col] = buf[k * B + col];
-    }
-}
+};
 
 template <typename T, int DIR>
-__global__ void __launch_bounds__(FFT_THREADS) fft_strided(Specs<cplx_t<T>> data, int nbatch, Strided s, Radices rd,
+__global__ void __launch_bounds__(FFT_THREADS, (sizeof(T) == 4 ? 3 : 2)) fft_strided(Specs<cplx_t<T>> data, int nbatch, Strided s, Radices rd,
                                                             int B) {
     typedef cplx_t<T> C;
     extern __shared__ unsigned char smem_raw[];
@@ -396,10 +446,7 @@ __global__ void __launch_bounds__(FFT_THREADS) fft_strided(Specs<cplx_t<T>> data
         const int o = (int)(r / ctiles), c0 = (int)(r % ctiles) * B;
         const int cols = min(B, s.ncols - c0);
         C* g = data.p[bi] + (int64_t)o * s.os + c0;
-        load_tile(bufa, g, s, B, cols);
-        __syncthreads();
-        C* res = fft_lines<C, DIR>(bufa, bufb, s.n, B, B, rd, tw, 1);
-        store_tile(g, res, s, B, cols);
+        fft_lines_through<C, DIR>(TileIn<C>{g, s.ls, cols}, TileOut<C>{g, s.ls, cols}, bufa, bufb, s.n, B, B, rd, tw, 1);
         __syncthreads();
     }
 }
@@ -490,7 +537,7 @@ __device__ __forceinline__ double2 kmultiplier(const KOp& op, int o, int ix, int
 }
 
 template <typename T>
-__global__ void __launch_bounds__(FFT_THREADS) fft_x_fused(Specs<cplx_t<T>> in, int nin, Specs<cplx_t<T>> out,
+__global__ void __launch_bounds__(FFT_THREADS, (sizeof(T) == 4 ? 3 : 2)) fft_x_fused(Specs<cplx_t<T>> in, int nin, Specs<cplx_t<T>> out,
                                                             Dims dims, int pitch, Radices rd, int B, KOp op) {
     typedef cplx_t<T> C;
     extern __shared__ unsigned char smem_raw[];
@@ -501,12 +548,7 @@ __global__ void __launch_bounds__(FFT_THREADS) fft_x_fused(Specs<cplx_t<T>> in, 
     C* bufb = bufa + n0 * B;
     fill_twiddles(tw, n0);
     __syncthreads();
-    Strided s;
-    s.n = n0;
-    s.ls = (int64_t)n1 * pitch;
-    s.outer = n1;
-    s.os = pitch;
-    s.ncols = nh;
+    const int64_t ls = (int64_t)n1 * pitch;
     const int ctiles = (nh + B - 1) / B, lb = log2_of(B);
     const int64_t tiles_per = (int64_t)n1 * ctiles;
     const int64_t ntiles = tiles_per * nin;
@@ -516,11 +558,7 @@ __global__ void __launch_bounds__(FFT_THREADS) fft_x_fused(Specs<cplx_t<T>> in, 
         const int iy = (int)(r / ctiles), c0 = (int)(r % ctiles) * B;
         const int cols = min(B, nh - c0);
         const int64_t off = (int64_t)iy * pitch + c0;
-        load_tile(bufa, in.p[bi] + off, s, B, cols);
-        __syncthreads();
-        C* fwd = fft_lines<C, -1>(bufa, bufb, n0, B, B, rd, tw, 1);
-        // keep the spectrum: copy to `spec` (the other buffer becomes free)
-        for (int q = threadIdx.x; q < n0 * B; q += blockDim.x) spec[q] = fwd[q];
+        fft_lines_through<C, -1>(TileIn<C>{in.p[bi] + off, ls, cols}, LinesOut<C>{spec, B}, bufa, bufb, n0, B, B, rd, tw, 1);
         __syncthreads();
         for (int o = 0; o < op.nper; o++) {
             for (int q = threadIdx.x; q < n0 * B; q += blockDim.x) {
@@ -530,8 +568,8 @@ __global__ void __launch_bounds__(FFT_THREADS) fft_x_fused(Specs<cplx_t<T>> in, 
                 bufa[q] = cmake<C>((T)(m.x * (double)v.x - m.y * (double)v.y), (T)(m.x * (double)v.y + m.y * (double)v.x));
             }
             __syncthreads();
-            C* res = fft_lines<C, +1>(bufa, bufb, n0, B, B, rd, tw, 1);
-            store_tile(out.p[bi * op.nper + o] + off, res, s, B, cols);
+            fft_lines_through<C, +1>(LinesIn<C>{bufa, B}, TileOut<C>{out.p[bi * op.nper + o] + off, ls, cols}, bufb, bufa, n0, B,
+                                     B, rd, tw, 1);
             __syncthreads();
         }
     }
@@ -772,8 +810,8 @@ template <typename T> static void pad_pitch(Plan3* p) {
 
 // Lines per tile B (a power of two) of a mixed-radix kernel whose blocks of B lines need `need(B)` bytes of shared memory:
 // 16, or 8 where three blocks of 16 do not fit on an SM, fewer still while two do not.  Plane-parallel passes of 500 x 450 x
-// 300 in FP32: 5.55 ms, 6.84 with 16 lines wherever two blocks fit; 360^3 3.83 and 4.08; 250^3 in FP64 2.13 and 2.11; 8
-// lines already where four blocks do not fit cost 150 x 125 x 243 a hundredth.
+// 300 in FP32: 5.37 ms, 6.52 with 16 lines wherever two blocks fit; 100^3 in FP64 0.176 and 0.190; 250^3 1.87 either way;
+// a bound of 44 KB takes the k-space pass of 150 x 125 x 243 from 0.40 to 0.45 ms.
 template <typename Need> static int choose_B(const Need& need) {
     int B = 16;
     while (B > 8 && need(B) > (size_t)60 * 1024) B >>= 1;

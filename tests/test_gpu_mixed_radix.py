@@ -9,9 +9,10 @@ import pytest
 
 from _util import maxrel
 
-# strided passes take 16 lines up to 232 points in FP32 and 116 in FP64; 606 and 1018 = 2 x 509 fewer than 8 in FP64
+# strided passes take 16 lines up to 232 points in FP32 and 116 in FP64; 606 and 1018 = 2 x 509 fewer than 8 in FP64;
+# 121 and 509 begin with a prime above 8
 SHAPES = [(232, 234, 18), (234, 232, 22), (116, 118, 30), (118, 116, 25), (5, 3, 466), (3, 7, 235), (2, 3, 2),
-          (49, 121, 231), (6, 606, 50), (1018, 2, 10)]
+          (49, 121, 231), (6, 606, 50), (1018, 2, 10), (509, 3, 4), (4, 509, 6)]
 
 
 def test_quotients_by_multiplication():
