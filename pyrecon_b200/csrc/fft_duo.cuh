@@ -7,7 +7,7 @@
 // column, its order included, is that of pass_regs and the kernels of fft_tma.cuh: the same bits.
 //
 // Measured per nmesh-512 reconstruction of the local-line-of-sight iteration, against one column a thread:
-// k-space pass 4.29 -> 3.55 ms (3.0 TB/s), Hessian pass 3.80 -> 3.16 ms (3.1 TB/s), y forward 1.41 -> 1.19 and y inverse
+// k-space pass 4.29 -> 3.45 ms (3.1 TB/s), Hessian pass 3.80 -> 3.15 ms (3.1 TB/s), y forward 1.41 -> 1.18 and y inverse
 // 1.15 -> 0.98 ms (5.5 TB/s).  The strided pass is within a fifth of a copy; the other two are bound by issue slots and
 // shared memory (46 instructions a point and transform, issue slots 53 to 57 % busy, then stalls on shared-memory
 // results), not by DRAM.
