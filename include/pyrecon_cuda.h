@@ -284,6 +284,10 @@ PRC_API void prc_tune_clear(void);
  * PRC_FAULT_WAIT_TIMEOUT in the fault word and returns; out (device int) = 1 when the wait gave up. */
 PRC_API int prc_debug_wait_timeout(int64_t limit_ns, int* out, void* stream);
 
+/* Blocks an SM that the mixed-radix strided pass over lines of n points (2 <= n <= 2048) is launched with on the
+ * current device (0 on a bad argument; nothing is launched). */
+PRC_API int prc_debug_fft_strided_blocks(int32_t n, int mesh_bytes);
+
 /* ------------------------------------------------------------------------------------------
  * FFTs and the k-space steps (the numpy / pyfftw sites of pyrecon/mesh.py:974-1118 and the
  * algorithm modules).  Forward transforms are unnormalised; inverse ones divide by n0*n1*n2,

@@ -26,7 +26,9 @@
 #include <algorithm>
 #include <map>
 #include <mutex>
+#include <tuple>
 #include <type_traits>
+#include <limits.h>
 #include <math.h>
 #include <string.h>
 #include <stdlib.h>
@@ -1030,25 +1032,29 @@ static bool spectrum_map(CUtensorMap* m, const void* base, const Plan3& p, size_
                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// Persistent grid: as many CTAs as fit on the device at once (occupancy of this kernel), at most
-// one per tile.
+// Persistent grid: as many CTAs as fit on the device at once (occupancy of this launch), at most one per tile.
 template <typename K> static int resident_grid(K kern, int threads, size_t smem, int64_t ntiles) {
-    // occupancy of (kernel, device), looked up once
+    // occupancy of (kernel, device, threads, shared memory), looked up once: a mixed-radix kernel's shared memory differs
+    // from one line length, tile width or number of inputs to the next (with the first launch's blocks kept for all, the
+    // six-input inverse z pass of a local-line-of-sight reconstruction had a third of its blocks in a second wave: three
+    // iterations at 300^3 in FP32 15.80 ms, 14.12 with its own)
+    typedef std::tuple<const void*, int, int, size_t> Key;
     static std::mutex mu;
-    static std::map<std::pair<const void*, int>, int> known;
+    static std::map<Key, int> known;
     int dev = 0;
     cudaGetDevice(&dev);
+    const Key key((const void*)kern, dev, threads, smem);
     int per_sm = 0;
     {
         std::lock_guard<std::mutex> lock(mu);
-        auto it = known.find({(const void*)kern, dev});
+        auto it = known.find(key);
         if (it != known.end()) per_sm = it->second;
     }
     if (per_sm == 0) {
         if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem) != cudaSuccess || per_sm < 1)
             per_sm = 1;
         std::lock_guard<std::mutex> lock(mu);
-        known[{(const void*)kern, dev}] = per_sm;
+        known[key] = per_sm;
     }
     const int64_t cap = (int64_t)device_sm_count() * per_sm;
     return (int)std::max<int64_t>(1, std::min<int64_t>(ntiles, cap));
@@ -1317,6 +1323,22 @@ template <typename T> struct FFTLaunch {
     typedef cplx_t<T> C;
     static constexpr size_t CS = sizeof(C);
 
+    // Lines per tile of the mixed-radix strided pass over lines of n points, and its shared memory.
+    static int strided_lines(int n, size_t* smem) {
+        auto need = [&](int b) { return (size_t)(2 * n * b + n) * CS; };
+        const int B = choose_B(need);
+        *smem = need(B);
+        return B;
+    }
+
+    // Blocks an SM that its launches count on.
+    static int strided_blocks(int n) {
+        size_t smem;
+        strided_lines(n, &smem);
+        cudaFuncSetAttribute(fft_strided<T, -1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        return resident_grid(fft_strided<T, -1>, FFT_THREADS, smem, INT_MAX) / device_sm_count();
+    }
+
     template <typename TIN>
     static int z_r2c(const Plan3& p, const void* const* in, C* const* out, int nb, cudaStream_t st) {
         if (p.dims.n[2] % 2 == 0 && fast_len(p.dims.n[2] / 2) && !getenv_generic()) {
@@ -1389,9 +1411,8 @@ template <typename T> struct FFTLaunch {
             s.os = p.pitch;
         }
         s.ncols = nh;
-        auto need = [&](int b) { return (size_t)(2 * s.n * b + s.n) * CS; };
-        const int B = choose_B(need);
-        const size_t smem = need(B);
+        size_t smem;
+        const int B = strided_lines(s.n, &smem);
         Specs<C> sp;
         for (int i = 0; i < nb; i++) sp.p[i] = data[i];
         cudaFuncSetAttribute(fft_strided<T, DIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -1844,6 +1865,11 @@ int prc_debug_wait_timeout(int64_t limit_ns, int* out, void* stream) {
     PRC_LAUNCH("debug_wait_timeout", st, debug_wait_timeout<<<1, 32, 0, st>>>((uint64_t)limit_ns, 256u, out));
     PRC_CHECK_LAUNCH();
     return PRC_OK;
+}
+
+int prc_debug_fft_strided_blocks(int32_t n, int mesh_bytes) {
+    if (n < 2 || n > MAX_FFT_N || (mesh_bytes != 4 && mesh_bytes != 8)) return 0;
+    return mesh_bytes == 4 ? FFTLaunch<float>::strided_blocks(n) : FFTLaunch<double>::strided_blocks(n);
 }
 
 int prc_fft_supported(const int32_t nmesh[3]) {
