@@ -1084,7 +1084,10 @@ template <int S0> struct StageCount {
 template <typename T, int N> struct StridedTmaB {
     static constexpr int B0 = PRC_TMA_STRIDED_B == 0 ? StridedCfg<T, N>::B
                                                      : (sizeof(T) == 4 ? PRC_TMA_STRIDED_B : PRC_TMA_STRIDED_B / 2);
-    static constexpr int value = (N / 8) * B0 <= 1024 ? B0 : 1024 / (N / 8);
+    static constexpr int B1 = (N / 8) * B0 <= 1024 ? B0 : 1024 / (N / 8);
+    // half as many where two stages and the twiddles do not fit beside each other (FP64 lines of 1024 points: 272 KB with
+    // 128-byte rows)
+    static constexpr int value = (size_t)(2 * B1 + 1) * N * sizeof(cplx_t<T>) + 64 <= 227 * 1024 ? B1 : B1 / 2;
 };
 
 template <typename T, int N> struct StridedTmaCfg {
@@ -1092,6 +1095,7 @@ template <typename T, int N> struct StridedTmaCfg {
     static constexpr int THREADS = (N / 8) * B;
     static constexpr int S = StageCount<(int)(PRC_TMA_STAGE_KB * 1024 / fast::TileShape<T, N, B>::BYTES)>::value;
     static constexpr size_t SMEM = fast::TmaSmem<T, N, B, S, fast::StridedPP<T, N, B, S>::value ? 1 : 0>::BYTES;
+    static_assert(SMEM <= 227 * 1024, "a strided tile's stages fit on an SM");
 };
 
 // Pairs of columns a tile and blocks an SM of the FP32 passes on pairs of columns (fft_duo.cuh): about 16 warps an SM
@@ -1156,6 +1160,7 @@ template <typename T, int N> struct KSpaceTmaCfg {
     static constexpr int S = 2;
     static constexpr bool PP = fast::KSpacePP<T, N, B, S, LEAN>::value;
     static constexpr size_t SMEM = fast::TmaSmem<T, N, B, S, PP ? 2 : 1, PP ? fast::PadFirst<T, B>::value : 0>::BYTES;
+    static_assert(SMEM <= 227 * 1024, "a k-space tile's stages fit on an SM");
 };
 
 template <typename T> struct FastXTma {
@@ -1233,6 +1238,7 @@ template <typename T, int N> struct HessTmaCfg {
     static constexpr int S = PP ? PRC_HESS_PP_S
                                 : StageCount<(int)(PRC_TMA_STAGE_KB * 1024 / fast::TileShape<T, N, B>::BYTES)>::value;
     static constexpr size_t SMEM = fast::TmaSmem<T, N, B, S, PP ? 1 : 0, PP ? PADX : 0>::BYTES;
+    static_assert(SMEM + 2 * N * sizeof(T) <= 227 * 1024, "a Hessian tile's stages and tables fit on an SM");
 };
 
 template <typename T> struct FastHessTma {
