@@ -284,6 +284,10 @@ PRC_API void prc_tune_clear(void);
  * PRC_FAULT_WAIT_TIMEOUT in the fault word and returns; out (device int) = 1 when the wait gave up. */
 PRC_API int prc_debug_wait_timeout(int64_t limit_ns, int* out, void* stream);
 
+/* Copies that a block of the FFT passes re-arming their stages one unit late waits for when the wait of `unit` (from 0)
+ * runs out, of `stages` stages: all that may still be in flight (host arithmetic, the kernels' own function). */
+PRC_API int prc_debug_units_in_flight(int64_t unit, int stages);
+
 /* Blocks an SM that the mixed-radix strided pass over lines of n points (2 <= n <= 2048) is launched with on the
  * current device (0 on a bad argument; nothing is launched). */
 PRC_API int prc_debug_fft_strided_blocks(int32_t n, int mesh_bytes);

@@ -1873,6 +1873,10 @@ int prc_debug_wait_timeout(int64_t limit_ns, int* out, void* stream) {
     return PRC_OK;
 }
 
+int prc_debug_units_in_flight(int64_t unit, int stages) {
+    return unit < 0 || stages < 1 ? 0 : fast::late_units(unit, stages);
+}
+
 int prc_debug_fft_strided_blocks(int32_t n, int mesh_bytes) {
     if (n < 2 || n > MAX_FFT_N || (mesh_bytes != 4 && mesh_bytes != 8)) return 0;
     return mesh_bytes == 4 ? FFTLaunch<float>::strided_blocks(n) : FFTLaunch<double>::strided_blocks(n);

@@ -368,7 +368,7 @@ __global__ void __launch_bounds__(N / 8 * BP, MINB)
         const int st = (int)(j % S);
         const bool ok = prc::tma::wait(&bars[st], (uint32_t)((j / S) & 1));
         if (__syncthreads_or(!ok)) {
-            if (tid == 0) drain<S>(bars, j, ntiles);
+            if (tid == 0) drain<S>(bars, j, ntiles, late_units(j, S));
             return;
         }
         // every thread is past tile j - 1, whose stage served the second exchange: it takes tile j - 1 + S
@@ -474,7 +474,7 @@ __global__ void __launch_bounds__(N / 8 * BP, MINB)
                 if (failed) {
                     if (tid == 0) {
                         atomicOr(&prc::g_fault, prc::tma::FAULT_WAIT_TIMEOUT);
-                        for (int d = 0; d < S - 1; d++) {      // units u .. u + S - 2 may be in flight
+                        for (int d = 0; d < late_units(u, S); d++) {
                             const int64_t uu = u + d;
                             if ((int64_t)blockIdx.x + (uu / 6) * gridDim.x >= ntiles) break;
                             prc::tma::wait(&bars[uu % S], (uint32_t)((uu / S) & 1));

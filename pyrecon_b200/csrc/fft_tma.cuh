@@ -54,12 +54,17 @@ __device__ __forceinline__ TileAt tile_at(int64_t tile, int64_t tiles_per, int c
     return a;
 }
 
+// Copies that may be in flight when the wait of unit u runs out, in a kernel that re-arms a stage one unit late (unit u,
+// once every thread is past unit u - 1, sends for unit u - 1 + S): the S of the prologue at unit 0, units u .. u + S - 2
+// later.
+__host__ __device__ constexpr int late_units(int64_t u, int S) { return u == 0 ? S : S - 1; }
+
 // Called by thread 0 after a wait ran out at local step j: wait (bounded) for the copies still in
-// flight, those of steps j .. j + S - 1, so none lands after the CTA has exited.
+// flight, those of steps j .. j + count - 1, so none lands after the CTA has exited.
 template <int S>
-__device__ __forceinline__ void drain(uint64_t* bars, int64_t j, int64_t ntiles) {
+__device__ __forceinline__ void drain(uint64_t* bars, int64_t j, int64_t ntiles, int count = S) {
     atomicOr(&prc::g_fault, prc::tma::FAULT_WAIT_TIMEOUT);
-    for (int d = 0; d < S; d++) {
+    for (int d = 0; d < count; d++) {
         const int64_t jj = j + d;
         if ((int64_t)blockIdx.x + jj * gridDim.x >= ntiles) break;
         prc::tma::wait(&bars[jj % S], (uint32_t)((jj / S) & 1));
@@ -599,8 +604,8 @@ __global__ void __launch_bounds__(N / 8 * B, (MinBlocks<T, N / 8 * B, MINB>::val
                 if (failed) {
                     if (tid == 0) {
                         atomicOr(&prc::g_fault, prc::tma::FAULT_WAIT_TIMEOUT);
-                        // units u .. u + S - 1 (u + S - 2 under PP) were issued and may be in flight
-                        for (int d = 0; d < (PP ? S - 1 : S); d++) {
+                        // without PP a stage is re-armed by the unit that read it: S units in flight
+                        for (int d = 0; d < (PP ? late_units(u, S) : S); d++) {
                             const int64_t uu = u + d;
                             if ((int64_t)blockIdx.x + (uu / 6) * gridDim.x >= ntiles) break;
                             prc::tma::wait(&bars[uu % S], (uint32_t)((uu / S) & 1));
