@@ -605,11 +605,14 @@ __global__ void __launch_bounds__(N / 8 * B, (MinBlocks<T, N / 8 * B, MINB>::val
                     if (tid == 0) {
                         atomicOr(&prc::g_fault, prc::tma::FAULT_WAIT_TIMEOUT);
                         // without PP a stage is re-armed by the unit that read it: S units in flight
-                        for (int d = 0; d < (PP ? late_units(u, S) : S); d++) {
+                        for (int d = 0; d < (PP ? late_units(1, S) : S); d++) {
                             const int64_t uu = u + d;
                             if ((int64_t)blockIdx.x + (uu / 6) * gridDim.x >= ntiles) break;
                             prc::tma::wait(&bars[uu % S], (uint32_t)((uu / S) & 1));
                         }
+                        // late_units(0, S): one more (as the loop's bound it costs the FP64 kernel 4 to 8 registers and
+                        // a block an SM, 0.42 -> 0.44 ms for three iterations at 128^3)
+                        if (PP && u == 0) prc::tma::wait(&bars[S - 1], 0);
                     }
                     return;
                 }
