@@ -1118,17 +1118,25 @@ template <int N> struct DuoCfg {
         return (int)std::max<size_t>(1, std::min<size_t>((226 * 1024) / (smem + 1024), 512 / threads));
     }
     static constexpr int KMINB = fit(KSMEM, KTHREADS), SMINB = fit(SSMEM, STHREADS), HMINB = fit(HSMEM, KTHREADS);
+    // Lines of 64 and 128 points keep both kernels: a launch whose tiles come to fewer than 8 warps an SM with two columns a
+    // thread runs one column a thread, twice the warps to wait with.  Plane-parallel passes (one column, two): 64^3 32.7
+    // and 37.8 us, 64 x 96 x 64 37.7 and 42.0 (k-space 3.2 warps an SM), 128 x 64 x 128 43.6 and 47.2 (7.8); three local
+    // iterations of 256 x 64 x 64 195 and 187 us (Hessian 8.6 warps an SM), of 64 x 64 x 512 248 and 224 (14).
+    static constexpr bool CHOOSE = N <= 128;
+    static bool fills(int64_t ntiles, int threads) {
+        return !CHOOSE || ntiles * threads >= (int64_t)8 * 32 * device_sm_count();
+    }
 };
 
 template <typename T, int DIR> struct FastStridedTma {
     template <int N> struct K {
-        static int run(const Plan3& p, Specs<cplx_t<T>> sp, int nb, Strided s, int axis, const char* name,
-                       double bytes, cudaStream_t st) {
-            constexpr bool duo = sizeof(T) == 4 && DuoCfg<N>::OK;
+        template <bool DUO>
+        static int go(const Plan3& p, Specs<cplx_t<T>> sp, int nb, Strided s, int axis, const char* name, double bytes,
+                      cudaStream_t st) {
             typedef StridedTmaCfg<T, N> cfg;
-            constexpr int B = duo ? 2 * DuoCfg<N>::SBP : cfg::B;
-            constexpr int THREADS = duo ? DuoCfg<N>::STHREADS : cfg::THREADS;
-            constexpr size_t SMEM = duo ? DuoCfg<N>::SSMEM : cfg::SMEM;
+            constexpr int B = DUO ? 2 * DuoCfg<N>::SBP : cfg::B;
+            constexpr int THREADS = DUO ? DuoCfg<N>::STHREADS : cfg::THREADS;
+            constexpr size_t SMEM = DUO ? DuoCfg<N>::SSMEM : cfg::SMEM;
             typedef fast::TileShape<T, N, B> TS;
             tma::Maps maps;
             for (int i = 0; i < nb; i++)
@@ -1143,8 +1151,18 @@ template <typename T, int DIR> struct FastStridedTma {
                 PRC_CHECK_LAUNCH();
                 return PRC_OK;
             };
-            if constexpr (duo) return launch(fast::strided_duo<N, DuoCfg<N>::SBP, DuoCfg<N>::S, DIR, DuoCfg<N>::SMINB>);
+            if constexpr (DUO) return launch(fast::strided_duo<N, DuoCfg<N>::SBP, DuoCfg<N>::S, DIR, DuoCfg<N>::SMINB>);
             else return launch(fast::strided_tma<T, N, cfg::B, cfg::S, DIR>);
+        }
+        static int run(const Plan3& p, Specs<cplx_t<T>> sp, int nb, Strided s, int axis, const char* name,
+                       double bytes, cudaStream_t st) {
+            typedef DuoCfg<N> duo;
+            if constexpr (sizeof(T) == 4 && duo::OK) {
+                const int64_t ntiles = (int64_t)s.outer * ((s.ncols + 2 * duo::SBP - 1) / (2 * duo::SBP)) * nb;
+                if (duo::fills(ntiles, duo::STHREADS)) return go<true>(p, sp, nb, s, axis, name, bytes, st);
+            }
+            if constexpr (sizeof(T) == 8 || !duo::OK || duo::CHOOSE) return go<false>(p, sp, nb, s, axis, name, bytes, st);
+            else return PRC_ERR_UNSUPPORTED;      // not reached
         }
     };
 };
@@ -1165,22 +1183,21 @@ template <typename T, int N> struct KSpaceTmaCfg {
 
 template <typename T> struct FastXTma {
     template <int N> struct K {
-        template <int KT>
-        static int go(Specs<cplx_t<T>> si, int nin, Specs<cplx_t<T>> so, const Plan3& p, KOp op, double bytes,
-                      cudaStream_t st) {
-            constexpr bool duo = sizeof(T) == 4 && DuoCfg<N>::K_OK && (KT == KOP_GAUSS || KT == KOP_PP || KT == KOP_PSI || KT == KOP_HESS3);
-            constexpr int B = duo ? 2 * DuoCfg<N>::KBP : KSpaceTmaCfg<T, N>::B;
-            constexpr int THREADS = duo ? DuoCfg<N>::KTHREADS : KSpaceTmaCfg<T, N>::THREADS;
-            constexpr size_t SMEM = duo ? DuoCfg<N>::KSMEM : KSpaceTmaCfg<T, N>::SMEM;
+        template <int KT, bool DUO>
+        static int launch(Specs<cplx_t<T>> si, int nin, Specs<cplx_t<T>> so, const Plan3& p, KOp op, double bytes,
+                          cudaStream_t st) {
+            constexpr int B = DUO ? 2 * DuoCfg<N>::KBP : KSpaceTmaCfg<T, N>::B;
+            constexpr int THREADS = DUO ? DuoCfg<N>::KTHREADS : KSpaceTmaCfg<T, N>::THREADS;
+            constexpr size_t SMEM = DUO ? DuoCfg<N>::KSMEM : KSpaceTmaCfg<T, N>::SMEM;
             typedef fast::TileShape<T, N, B> TS;
             tma::Maps maps;
             for (int i = 0; i < nin; i++)
                 if (!spectrum_map(&maps.m[i], si.p[i], p, sizeof(cplx_t<T>), B, 1, TS::BOXL)) return TMA_UNAVAILABLE;
-            if (duo)         // pairs of columns are stored as 16-byte vectors
+            if (DUO)         // pairs of columns are stored as 16-byte vectors
                 for (int i = 0; i < nin * op.nper; i++)
                     if (((uintptr_t)so.p[i] & 15) != 0) return TMA_UNAVAILABLE;
             const int64_t ntiles = (int64_t)p.dims.n[1] * ((p.nh + B - 1) / B) * nin;
-            auto launch = [&](auto kern) {
+            auto with = [&](auto kern) {
                 cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM);
                 PRC_LAUNCH_B("fft_x_kspace", st, bytes,
                              kern<<<resident_grid(kern, THREADS, SMEM, ntiles), THREADS, SMEM, st>>>(maps, nin, so, p.dims,
@@ -1188,8 +1205,23 @@ template <typename T> struct FastXTma {
                 PRC_CHECK_LAUNCH();
                 return PRC_OK;
             };
-            if constexpr (duo) return launch(fast::x_kspace_duo<N, DuoCfg<N>::KBP, KT, DuoCfg<N>::KMINB>);
-            else return launch(fast::x_kspace_tma<T, N, B, KSpaceTmaCfg<T, N>::S, KT, KSpaceTmaCfg<T, N>::LEAN>);
+            if constexpr (DUO) return with(fast::x_kspace_duo<N, DuoCfg<N>::KBP, KT, DuoCfg<N>::KMINB>);
+            else return with(fast::x_kspace_tma<T, N, B, KSpaceTmaCfg<T, N>::S, KT, KSpaceTmaCfg<T, N>::LEAN>);
+        }
+        template <int KT>
+        static int go(Specs<cplx_t<T>> si, int nin, Specs<cplx_t<T>> so, const Plan3& p, KOp op, double bytes,
+                      cudaStream_t st) {
+            typedef DuoCfg<N> duo;
+            // the plane-parallel step divides twice a point: at 64 points a pair's sixteen divisions a thread are a loss at
+            // any size (64 x 512 x 64 76.0 and 81.1 us, 64 x 1024 x 64 134 and 132, 124 with pairs in the y pass alone)
+            constexpr bool use = sizeof(T) == 4 && duo::K_OK &&
+                                 (KT == KOP_GAUSS || (KT == KOP_PP && N >= 128) || KT == KOP_PSI || KT == KOP_HESS3);
+            if constexpr (use) {
+                const int64_t ntiles = (int64_t)p.dims.n[1] * ((p.nh + 2 * duo::KBP - 1) / (2 * duo::KBP)) * nin;
+                if (duo::fills(ntiles, duo::KTHREADS)) return launch<KT, true>(si, nin, so, p, op, bytes, st);
+            }
+            if constexpr (!use || duo::CHOOSE) return launch<KT, false>(si, nin, so, p, op, bytes, st);
+            else return PRC_ERR_UNSUPPORTED;      // not reached
         }
         static int run(const Plan3& p, Specs<cplx_t<T>> si, int nin, Specs<cplx_t<T>> so, KOp op, double bytes,
                        cudaStream_t st) {
@@ -1244,47 +1276,50 @@ template <typename T, int N> struct HessTmaCfg {
 template <typename T> struct FastHessTma {
     template <int N> struct K {
         typedef HessTmaCfg<T, N> cfg;
-        // probe: only check that the tensor maps can be made (nothing is launched)
-        static int run(const Plan3& p, cplx_t<T>* const* d, cplx_t<T>* const* o, fast::HessGeom h, cudaStream_t st,
-                       bool probe) {
-            constexpr bool use_duo = sizeof(T) == 4 && DuoCfg<N>::OK;
-            constexpr int B = use_duo ? 2 * DuoCfg<N>::KBP : cfg::B;
+        template <bool DUO>
+        static int go(const Plan3& p, cplx_t<T>* const* d, cplx_t<T>* const* o, fast::HessGeom h, cudaStream_t st,
+                      bool probe) {
+            constexpr int B = DUO ? 2 * DuoCfg<N>::KBP : cfg::B;
+            constexpr int THREADS = DUO ? DuoCfg<N>::KTHREADS : cfg::THREADS;
+            // one column a thread: + the x1 and k_y tables
+            constexpr size_t SMEM = DUO ? DuoCfg<N>::HSMEM : cfg::SMEM + 2 * N * sizeof(T);
             typedef fast::TileShape<T, N, B> TS;
             tma::Maps maps;
             for (int i = 0; i < 3; i++)
                 if (!spectrum_map(&maps.m[i], d[i], p, sizeof(cplx_t<T>), B, TS::BOXL, 1) ||
-                    (use_duo && ((uintptr_t)o[i] & 15) != 0))
+                    (DUO && ((uintptr_t)o[i] & 15) != 0))
                     return TMA_UNAVAILABLE;
             if (probe) return PRC_OK;
             Specs<cplx_t<T>> so;
             for (int i = 0; i < 3; i++) so.p[i] = o[i];
             Strided s;
-            s.n = p.dims.n[1];
+            s.n = N;
             s.ls = p.pitch;
             s.outer = p.dims.n[0];
             s.os = (int64_t)p.dims.n[1] * p.pitch;
             s.ncols = p.nh;
             const int64_t ntiles = (int64_t)s.outer * ((s.ncols + B - 1) / B);
             const double bytes = 6.0 * spectrum_values(p) * sizeof(cplx_t<T>);
-            if constexpr (use_duo) {
-                typedef DuoCfg<N> duo;
-                auto kern = fast::y_hessian_duo<N, duo::KBP, duo::S, duo::HMINB>;
-                cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)duo::HSMEM);
+            auto launch = [&](auto kern) {
+                cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM);
                 PRC_LAUNCH_B("fft_y_inv_hessian", st, bytes,
-                             kern<<<resident_grid(kern, duo::KTHREADS, duo::HSMEM, ntiles), duo::KTHREADS, duo::HSMEM, st>>>(
-                                 maps, so, s, h));
+                             kern<<<resident_grid(kern, THREADS, SMEM, ntiles), THREADS, SMEM, st>>>(maps, so, s, h));
                 PRC_CHECK_LAUNCH();
                 return PRC_OK;
-            } else {
-            auto kern = fast::y_hessian_tma<T, N, cfg::B, cfg::S, cfg::MINB, cfg::PP>;
-            const size_t smem = cfg::SMEM + 2 * N * sizeof(T);     // + the x1 and k_y tables
-            cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            PRC_LAUNCH_B("fft_y_inv_hessian", st, bytes,
-                         kern<<<resident_grid(kern, cfg::THREADS, smem, ntiles), cfg::THREADS, smem, st>>>(
-                             maps, so, s, h));
-            PRC_CHECK_LAUNCH();
-            return PRC_OK;
+            };
+            if constexpr (DUO) return launch(fast::y_hessian_duo<N, DuoCfg<N>::KBP, DuoCfg<N>::S, DuoCfg<N>::HMINB>);
+            else return launch(fast::y_hessian_tma<T, N, cfg::B, cfg::S, cfg::MINB, cfg::PP>);
+        }
+        // probe: only check that the tensor maps can be made (nothing is launched)
+        static int run(const Plan3& p, cplx_t<T>* const* d, cplx_t<T>* const* o, fast::HessGeom h, cudaStream_t st,
+                       bool probe) {
+            typedef DuoCfg<N> duo;
+            if constexpr (sizeof(T) == 4 && duo::OK) {
+                const int64_t ntiles = (int64_t)p.dims.n[0] * ((p.nh + 2 * duo::KBP - 1) / (2 * duo::KBP));
+                if (duo::fills(ntiles, duo::KTHREADS)) return go<true>(p, d, o, h, st, probe);
             }
+            if constexpr (sizeof(T) == 8 || !duo::OK || duo::CHOOSE) return go<false>(p, d, o, h, st, probe);
+            else return PRC_ERR_UNSUPPORTED;      // not reached
         }
     };
 };
