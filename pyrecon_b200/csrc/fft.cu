@@ -811,12 +811,12 @@ template <typename T> static void pad_pitch(Plan3* p) {
 }
 
 // Lines per tile B (a power of two) of a mixed-radix kernel whose blocks of B lines need `need(B)` bytes of shared memory:
-// 16, or 8 where three blocks of 16 do not fit on an SM, fewer still while two do not.  Plane-parallel passes of 500 x 450 x
-// 300 in FP32: 5.37 ms, 6.52 with 16 lines wherever two blocks fit; 100^3 in FP64 0.176 and 0.190; 250^3 1.87 either way;
-// a bound of 44 KB takes the k-space pass of 150 x 125 x 243 from 0.40 to 0.45 ms.
-template <typename Need> static int choose_B(const Need& need) {
+// 16 up to `wide` bytes, 8 above, fewer still while two blocks do not fit on an SM (100 KB).  Plane-parallel passes of 500 x
+// 450 x 300 in FP32: 5.37 ms, 6.52 with 16 lines wherever two blocks fit; 100^3 in FP64 0.176 and 0.190; 250^3 1.87 either
+// way; a bound of 44 KB takes the k-space pass of 150 x 125 x 243 from 0.40 to 0.45 ms.
+template <typename Need> static int choose_B(const Need& need, size_t wide = (size_t)60 * 1024) {
     int B = 16;
-    while (B > 8 && need(B) > (size_t)60 * 1024) B >>= 1;
+    while (B > 8 && need(B) > wide) B >>= 1;
     while (B > 1 && need(B) > (size_t)100 * 1024) B >>= 1;
     return B;
 }
@@ -1522,7 +1522,9 @@ template <typename T> struct FFTLaunch {
         auto need = [&](int b) {
             return (size_t)(2 * L * row_pitch(b) + n2) * CS + (size_t)nin * b * n2 * sizeof(T);
         };
-        const int B = choose_B(need);
+        // FP64: two blocks an SM at 124 registers, however small; 8 lines took three local iterations at 96^3 from 0.476 to
+        // 0.531 ms, plane-parallel passes at 150^3 from 0.436 to 0.466
+        const int B = choose_B(need, (size_t)(sizeof(T) == 4 ? 60 : 100) * 1024);
         const size_t smem = need(B);
         Specs<C> si;
         for (int i = 0; i < nin; i++) si.p[i] = in[i];
