@@ -241,51 +241,80 @@ __device__ __forceinline__ void quad_load(const V* __restrict__ v, const Stencil
 
 namespace prc {
 
-// U, W, q and P (op_terms) of a quad's cells 2 j, 2 j + 1 from its columns.  The axis modes leave out terms that are exact
-// zeros: W is one product, whose factors s_a and v+a + v-a are returned in (W, wf) for the caller to multiply.
-template <int MODE, typename T, typename P2 = typename Pair<T>::T>
-__device__ __forceinline__ void quad_terms(const QuadCols<T>& Q, const OpCoef<T>& k, const XYCoef<T>& c, int z0, int j,
-                                           P2& U, P2& W, P2& wf, P2& q, P2& PP) {
-    constexpr bool LOCAL = MODE == MG_LOCAL;
-    typedef Pair<T> P;
-    const int i = 2 * j;
-    const P2 p2 = P::make(z_p2<LOCAL>(k, z0 + i), z_p2<LOCAL>(k, z0 + i + 1)), s2 = P::mul(p2, p2);
-    const P2 xp = P::make(Q.XP[i + 1], Q.XP[i + 2]), xm = P::make(Q.XM[i + 1], Q.XM[i + 2]);
-    const P2 yp = P::make(Q.YP[i + 1], Q.YP[i + 2]), ym = P::make(Q.YM[i + 1], Q.YM[i + 2]);
-    const P2 zp = P::make(Q.c[i + 2], Q.c[i + 3]), zm = P::make(Q.c[i], Q.c[i + 1]);
-    if constexpr (MODE >= MG_AXIS0) {
-        const P2 Sx = P::add(xp, xm), Sy = P::add(yp, ym), Sz = P::add(zp, zm);
-        U = P::fma(both(k.ih0), Sx, P::mul(both(k.ih1), Sy));
-        U = P::fma(both(k.ih2), Sz, U);
-        W = MODE == MG_AXIS0 ? Sx : (MODE == MG_AXIS1 ? Sy : Sz);
-        wf = MODE == MG_AXIS0 ? both(c.s0) : (MODE == MG_AXIS1 ? both(c.s1) : s2);
-        q = P::fma(both(k.h22), s2, both(c.q01));
-        PP = P::add(both(c.P01), s2);
-    } else {
-        const P2 exy = P::sub(P::add(P::make(Q.PP[i], Q.PP[i + 1]), P::make(Q.MM[i], Q.MM[i + 1])),
-                              P::add(P::make(Q.MP[i], Q.MP[i + 1]), P::make(Q.PM[i], Q.PM[i + 1])));
-        const P2 exz = P::sub(P::add(P::make(Q.XP[i + 2], Q.XP[i + 3]), P::make(Q.XM[i], Q.XM[i + 1])),
-                              P::add(P::make(Q.XM[i + 2], Q.XM[i + 3]), P::make(Q.XP[i], Q.XP[i + 1])));
-        const P2 eyz = P::sub(P::add(P::make(Q.YP[i + 2], Q.YP[i + 3]), P::make(Q.YM[i], Q.YM[i + 1])),
-                              P::add(P::make(Q.YM[i + 2], Q.YM[i + 3]), P::make(Q.YP[i], Q.YP[i + 1])));
-        op_terms<LOCAL, P>(k, c, p2, s2, xp, xm, yp, ym, zp, zm, exy, exz, eyz, U, W, q, PP);
+// U, W, q and P (op_terms) of a quad's cell i from its columns, one cell at a time: pairs would start at an odd column, and
+// the moves and registers they cost (80 against 64 in the FP32 sweep: 512 x 512 x 8 9.3 and 8.7 us) take warps from kernels
+// that wait on memory.
+template <bool LOCAL, typename T>
+__device__ __forceinline__ void quad_terms(const QuadCols<T>& Q, const OpCoef<T>& k, const XYCoef<T>& c, int z0, int i,
+                                           T& U, T& W, T& q, T& PP) {
+    const T p2 = z_p2<LOCAL>(k, z0 + i), s2 = rn_mul(p2, p2);
+    const T exy = rn_sub(rn_add(Q.PP[i], Q.MM[i]), rn_add(Q.MP[i], Q.PM[i]));
+    const T exz = rn_sub(rn_add(Q.XP[i + 2], Q.XM[i]), rn_add(Q.XM[i + 2], Q.XP[i]));
+    const T eyz = rn_sub(rn_add(Q.YP[i + 2], Q.YM[i]), rn_add(Q.YM[i + 2], Q.YP[i]));
+    op_terms<LOCAL, One<T>>(k, c, p2, s2, Q.XP[i + 1], Q.XM[i + 1], Q.YP[i + 1], Q.YM[i + 1], Q.c[i + 2], Q.c[i], exy, exz, eyz,
+                            U, W, q, PP);
+}
+
+// U, W, q and P of the axis modes, which leave out terms that are exact zeros, and the damped-Jacobi values from them.  The
+// expressions are left to the compiler, for all four cells before the divisions: in pairs of cells, spelled out as op_terms,
+// they took 40 registers instead of 32 in the FP32 sweep and 70 instead of 64 in the FP64 one (a sweep at 256^3: FP32 33.8 us
+// and 37.3 in pairs, FP64 along y 78 and 95).
+template <int MODE, typename T>
+__device__ __forceinline__ void axis_terms(const QuadCols<T>& Q, const Stencil<T>& s, T (&U)[4], T (&W)[4], T (&qq)[4],
+                                           T (&P)[4]) {
+    const T ih0 = s.ih2[0], ih1 = s.ih2[1], ih2 = s.ih2[2];
+    const T p0 = s.losh[0], p1 = s.losh[1], p2 = s.losh[2];
+    const T s0 = p0 * p0, s1 = p1 * p1;
+    const T q01 = s.h2[0] * s0 + s.h2[1] * s1, P01 = s0 + s1;
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        const T s2 = p2 * p2;
+        const T xpv = Q.XP[k + 1], xmv = Q.XM[k + 1], ypv = Q.YP[k + 1], ymv = Q.YM[k + 1], zpv = Q.c[k + 2], zmv = Q.c[k];
+        U[k] = ih0 * (xpv + xmv) + ih1 * (ypv + ymv) + ih2 * (zpv + zmv);
+        if constexpr (MODE == MG_AXIS0) W[k] = s0 * (xpv + xmv);
+        else if constexpr (MODE == MG_AXIS1) W[k] = s1 * (ypv + ymv);
+        else W[k] = s2 * (zpv + zmv);
+        qq[k] = q01 + s.h2[2] * s2;
+        P[k] = P01 + s2;
+    }
+}
+// The same where v is identically zero.
+template <typename T>
+__device__ __forceinline__ void axis_zero_terms(const Stencil<T>& s, T (&U)[4], T (&W)[4], T (&qq)[4], T (&P)[4], T (&vc)[4]) {
+    const T p0 = s.losh[0], p1 = s.losh[1], p2 = s.losh[2];
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        const T s2 = p2 * p2;
+        qq[k] = s.h2[0] * p0 * p0 + s.h2[1] * p1 * p1 + s.h2[2] * s2;
+        P[k] = p0 * p0 + p1 * p1 + s2;
+        U[k] = W[k] = vc[k] = (T)0;
+    }
+}
+template <typename T> __device__ __forceinline__ T quotient(T a, T b) {
+    if constexpr (sizeof(T) == 4) return __fdividef(a, b);
+    else return a / b;
+}
+template <typename T>
+__device__ __forceinline__ void axis_blend(const Stencil<T>& s, T w, const T (&fv)[4], const T (&vc)[4], const T (&U)[4],
+                                           const T (&W)[4], const T (&qq)[4], const T (&P)[4], T (&o)[4]) {
+    const T sih = s.ih2[0] + s.ih2[1] + s.ih2[2];
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        const T jac = quotient<T>(qq[k] * (fv[k] + U[k]) + s.beta * W[k], (T)2 * (qq[k] * sih + s.beta * P[k]));
+        o[k] = vc[k] + w * (jac - vc[k]);
     }
 }
 
-// The damped-Jacobi values of a quad from its columns.
-template <int MODE, typename T>
+// The damped-Jacobi values of a quad from its columns (19-point operator).
+template <bool LOCAL, typename T>
 __device__ __forceinline__ void quad_jacobi(const QuadCols<T>& Q, const OpCoef<T>& k, T w, int x, int y, int z0,
                                             const T (&f)[4], T (&o)[4]) {
-    typedef Pair<T> P;
-    const XYCoef<T> c = xy_coef<MODE == MG_LOCAL>(k, x, y);
+    const XYCoef<T> c = xy_coef<LOCAL>(k, x, y);
 #pragma unroll
-    for (int j = 0; j < 2; j++) {
-        typename P::T U, W, wf, q, PP;
-        quad_terms<MODE>(Q, k, c, z0, j, U, W, wf, q, PP);
-        if (MODE >= MG_AXIS0) W = P::mul(wf, W);
-        const typename P::T r = op_jacobi<P>(k, P::make(f[2 * j], f[2 * j + 1]), P::make(Q.c[2 * j + 1], Q.c[2 * j + 2]), U, W,
-                                          q, PP, w);
-        o[2 * j] = r.x, o[2 * j + 1] = r.y;
+    for (int i = 0; i < 4; i++) {
+        T U, W, q, PP;
+        quad_terms<LOCAL>(Q, k, c, z0, i, U, W, q, PP);
+        o[i] = op_jacobi<One<T>>(k, f[i], Q.c[i + 1], U, W, q, PP, w);
     }
 }
 
@@ -320,10 +349,10 @@ template <typename T> __device__ __forceinline__ void store4(T* p, const T (&o)[
     }
 }
 
-// Damped-Jacobi sweep of four cells per thread: the axis modes, rows too long for march_kernel, and (zero_v)
-// every sweep from an identically zero v.
-// acc (optional): the sweep's result is added to it instead of being stored (OP_JACOBI_ADD).
-template <typename T, int MODE>
+// Damped-Jacobi sweep of four cells per thread: the axis modes, the 19-point ones where march_ok leaves them here (short
+// rows, small meshes), and (zero_v) every sweep from an identically zero v.
+// ADD: the sweep's result is added to acc instead of being stored (OP_JACOBI_ADD).
+template <typename T, int MODE, bool ADD>
 __global__ void __launch_bounds__(256) jacobi_sweep4(const T* __restrict__ v, const T* __restrict__ f,
                                                      T* __restrict__ vout, double* __restrict__ acc, Stencil<T> s, T w,
                                                      int zero_v) {
@@ -333,17 +362,27 @@ __global__ void __launch_bounds__(256) jacobi_sweep4(const T* __restrict__ v, co
     if (!quad_of(s.n, q)) return;
     const int64_t bo = batch_offset(s.n);
     v += bo, f += bo, vout += bo;
-    const OpCoef<T> k = op_coef<MODE == MG_LOCAL>(s);
     T fv[4], o[4];
     load4(f + q.c + q.z0, fv);
-    if (zero_v) {
-        quad_zero<MODE == MG_LOCAL>(k, w, q.x, q.y, q.z0, fv, o);
+    if constexpr (MODE >= MG_AXIS0) {
+        T U[4], W[4], qq[4], P[4], vc[4];
+        if (zero_v) {
+            axis_zero_terms(s, U, W, qq, P, vc);
+        } else {
+            QuadCols<T> Q;
+            quad_load<MODE>(v, s, q, Q);
+            axis_terms<MODE>(Q, s, U, W, qq, P);
+            load4(v + q.c + q.z0, vc);
+        }
+        axis_blend(s, w, fv, vc, U, W, qq, P, o);
+    } else if (zero_v) {
+        quad_zero<MODE == MG_LOCAL>(op_coef<MODE == MG_LOCAL>(s), w, q.x, q.y, q.z0, fv, o);
     } else {
         QuadCols<T> Q;
         quad_load<MODE>(v, s, q, Q);
-        quad_jacobi<MODE>(Q, k, w, q.x, q.y, q.z0, fv, o);
+        quad_jacobi<MODE == MG_LOCAL>(Q, op_coef<MODE == MG_LOCAL>(s), w, q.x, q.y, q.z0, fv, o);
     }
-    if (acc != nullptr) {
+    if constexpr (ADD) {
         double* a = acc + bo + q.c + q.z0;
         double t[4];
 #pragma unroll
@@ -483,7 +522,7 @@ __global__ void __launch_bounds__(TQ * TY, (sizeof(T) == 4 ? 6 : 4)) jacobi_swee
                 } else {
                     QuadCols<T> Q;
                     smem_cols<T, ZP>(lo, mid, hi, r + 1, 4 * k + 4, Q);
-                    quad_jacobi<LOCAL ? MG_LOCAL : MG_GLOBAL>(Q, kc, w, gx, gy, gz, fv, o);
+                    quad_jacobi<LOCAL>(Q, kc, w, gx, gy, gz, fv, o);
                 }
                 smem_store4(out + r * ZP, 4 * k + 4, o);
             }
@@ -503,7 +542,7 @@ __global__ void __launch_bounds__(TQ * TY, (sizeof(T) == 4 ? 6 : 4)) jacobi_swee
                 load4(f + at, fv);
                 QuadCols<T> Q;
                 smem_cols<T, ZP>(lo, mid, hi, r + 1, 4 * k + 8, Q);
-                quad_jacobi<LOCAL ? MG_LOCAL : MG_GLOBAL>(Q, kc, w, xo, gy, gz, fv, o);
+                quad_jacobi<LOCAL>(Q, kc, w, xo, gy, gz, fv, o);
                 if constexpr (sizeof(T) == 4) {
                     *(float4*)(vout + at) = make_float4(o[0], o[1], o[2], o[3]);
                 } else {
@@ -515,8 +554,8 @@ __global__ void __launch_bounds__(TQ * TY, (sizeof(T) == 4 ? 6 : 4)) jacobi_swee
     }
 }
 
-// r = f - A v of four cells per thread, evaluated in type A and stored as R: the axis modes, and rows too long for
-// march_kernel.
+// r = f - A v of four cells per thread, evaluated in type A and stored as R: the axis modes, and the 19-point ones where
+// march_ok leaves them here.
 template <typename A, typename R, int MODE>
 __global__ void __launch_bounds__(256) residual_kernel4(const A* __restrict__ v, const A* __restrict__ f,
                                                         R* __restrict__ r, Stencil<A> s) {
@@ -526,29 +565,34 @@ __global__ void __launch_bounds__(256) residual_kernel4(const A* __restrict__ v,
     if (!quad_of(s.n, q)) return;
     const int64_t bo = batch_offset(s.n);
     v += bo, f += bo, r += bo;
-    typedef Pair<A> P;
     QuadCols<A> Q;
-    A fv[4];
-    R o[4];
     quad_load<MODE>(v, s, q, Q);
-    load4(f + q.c + q.z0, fv);
-    const OpCoef<A> k = op_coef<MODE == MG_LOCAL>(s);
-    const XYCoef<A> c = xy_coef<MODE == MG_LOCAL>(k, q.x, q.y);
+    if constexpr (MODE >= MG_AXIS0) {
+        A U[4], W[4], qq[4], P[4], vc[4], fv[4];
+        axis_terms<MODE>(Q, s, U, W, qq, P);
+        load4(v + q.c + q.z0, vc);
+        load4(f + q.c + q.z0, fv);
+        const A sih2 = (A)2 * (s.ih2[0] + s.ih2[1] + s.ih2[2]);
 #pragma unroll
-    for (int j = 0; j < 2; j++) {
-        typename P::T U, W, wf, qq, PP;
-        quad_terms<MODE>(Q, k, c, q.z0, j, U, W, wf, qq, PP);
-        const typename P::T v2 = P::make(Q.c[2 * j + 1], Q.c[2 * j + 2]), f2 = P::make(fv[2 * j], fv[2 * j + 1]);
-        typename P::T t;
-        if constexpr (MODE >= MG_AXIS0 && sizeof(A) == 4) {
-            t = op_residual_from<P>(k, f2, v2, U, P::fma(wf, W, P::mul(P::mul(both((A)-2), PP), v2)), qq);
-        } else {
-            if (MODE >= MG_AXIS0) W = P::mul(wf, W);
-            t = op_residual<P>(k, f2, v2, U, W, qq, PP);
+        for (int k = 0; k < 4; k++) {
+            const A g = quotient<A>(s.beta, qq[k]);
+            const A x = vc[k];
+            r[q.c + q.z0 + k] = (R)((fv[k] + U[k] - sih2 * x) + g * (W[k] - (A)2 * P[k] * x));
         }
-        o[2 * j] = (R)t.x, o[2 * j + 1] = (R)t.y;
+    } else {
+        A fv[4];
+        R o[4];
+        load4(f + q.c + q.z0, fv);
+        const OpCoef<A> k = op_coef<MODE == MG_LOCAL>(s);
+        const XYCoef<A> c = xy_coef<MODE == MG_LOCAL>(k, q.x, q.y);
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            A U, W, qq, PP;
+            quad_terms<MODE == MG_LOCAL>(Q, k, c, q.z0, i, U, W, qq, PP);
+            o[i] = (R)op_residual<One<A>>(k, fv[i], Q.c[i + 1], U, W, qq, PP);
+        }
+        store4(r + q.c + q.z0, o);
     }
-    store4(r + q.c + q.z0, o);
 }
 
 // r = f - A v, evaluated in type A (double for the mixed-precision defect), stored as R.
@@ -570,13 +614,13 @@ __global__ void __launch_bounds__(256) residual_kernel(const V* __restrict__ v, 
 }
 
 // The quad kernels' instance for an operator form (mg_mode).
-template <typename T> static decltype(&jacobi_sweep4<T, MG_GLOBAL>) sweep4_kernel(int mode) {
+template <typename T, bool ADD> static decltype(&jacobi_sweep4<T, MG_GLOBAL, ADD>) sweep4_kernel(int mode) {
     switch (mode) {
-    case MG_LOCAL: return jacobi_sweep4<T, MG_LOCAL>;
-    case MG_AXIS0: return jacobi_sweep4<T, MG_AXIS0>;
-    case MG_AXIS1: return jacobi_sweep4<T, MG_AXIS1>;
-    case MG_AXIS2: return jacobi_sweep4<T, MG_AXIS2>;
-    default: return jacobi_sweep4<T, MG_GLOBAL>;
+    case MG_LOCAL: return jacobi_sweep4<T, MG_LOCAL, ADD>;
+    case MG_AXIS0: return jacobi_sweep4<T, MG_AXIS0, ADD>;
+    case MG_AXIS1: return jacobi_sweep4<T, MG_AXIS1, ADD>;
+    case MG_AXIS2: return jacobi_sweep4<T, MG_AXIS2, ADD>;
+    default: return jacobi_sweep4<T, MG_GLOBAL, ADD>;
     }
 }
 template <typename A, typename R> static decltype(&residual_kernel4<A, R, MG_GLOBAL>) residual4_kernel(int mode) {
@@ -987,7 +1031,7 @@ template <typename T> struct MGRunner {
                                  (launch_march<T, T, OP_JACOBI>(v, f, tmp, nullptr, s, (T)P.damping, count, st)));
             } else if (quad) {
                 PRC_LAUNCH_B(a != nullptr ? "mg_jacobi_add" : "mg_jacobi", st, bytes,
-                             launch_pdl(sweep4_kernel<T>(mg_mode(s)), gq.grid, gq.block, 0, st, v, f, tmp, a, s, (T)P.damping, z0));
+                             launch_pdl(a != nullptr ? sweep4_kernel<T, true>(mg_mode(s)) : sweep4_kernel<T, false>(mg_mode(s)), gq.grid, gq.block, 0, st, v, f, tmp, a, s, (T)P.damping, z0));
             } else {
                 PRC_LAUNCH_B("mg_jacobi", st, (double)N * sizeof(T) * (z0 ? 2 : 3),
                              launch_pdl(jacobi_sweep<T, T>, g.grid, g.block, 0, st, v, f, tmp, s, (T)P.damping, z0));
