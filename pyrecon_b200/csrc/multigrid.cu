@@ -566,6 +566,7 @@ __global__ void __launch_bounds__(256) residual_kernel4(const A* __restrict__ v,
     const int64_t bo = batch_offset(s.n);
     v += bo, f += bo, r += bo;
     QuadCols<A> Q;
+    R o[4];
     quad_load<MODE>(v, s, q, Q);
     if constexpr (MODE >= MG_AXIS0) {
         A U[4], W[4], qq[4], P[4], vc[4], fv[4];
@@ -577,11 +578,10 @@ __global__ void __launch_bounds__(256) residual_kernel4(const A* __restrict__ v,
         for (int k = 0; k < 4; k++) {
             const A g = quotient<A>(s.beta, qq[k]);
             const A x = vc[k];
-            r[q.c + q.z0 + k] = (R)((fv[k] + U[k] - sih2 * x) + g * (W[k] - (A)2 * P[k] * x));
+            o[k] = (R)((fv[k] + U[k] - sih2 * x) + g * (W[k] - (A)2 * P[k] * x));
         }
     } else {
         A fv[4];
-        R o[4];
         load4(f + q.c + q.z0, fv);
         const OpCoef<A> k = op_coef<MODE == MG_LOCAL>(s);
         const XYCoef<A> c = xy_coef<MODE == MG_LOCAL>(k, q.x, q.y);
@@ -591,8 +591,8 @@ __global__ void __launch_bounds__(256) residual_kernel4(const A* __restrict__ v,
             quad_terms<MODE == MG_LOCAL>(Q, k, c, q.z0, i, U, W, qq, PP);
             o[i] = (R)op_residual<One<A>>(k, fv[i], Q.c[i + 1], U, W, qq, PP);
         }
-        store4(r + q.c + q.z0, o);
     }
+    store4(r + q.c + q.z0, o);
 }
 
 // r = f - A v, evaluated in type A (double for the mixed-precision defect), stored as R.
