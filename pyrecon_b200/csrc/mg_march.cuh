@@ -378,28 +378,41 @@ __global__ void __launch_bounds__(MARCH_THREADS, 2)
     }
 }
 
+// Lanes a row of a march over rows of n2 cells: the power of two that computes the least, each segment's halo counted (a
+// segment that is the whole row has none); 0 where a row does not hold a tile.  cells: what a row then computes and stages.
+template <typename A> static int march_lanes(int n2, int* cells) {
+    constexpr int VZ = MarchVZ<A>::value;
+    int best = 0;
+    *cells = 0;
+    for (int lz = 32; lz >= 4; lz >>= 1) {
+        const int tz = lz * VZ, c = (n2 + tz - 1) / tz * (tz + 2 * VZ);
+        if (tz <= n2 && (best == 0 || c < *cells)) best = lz, *cells = c;
+    }
+    if (best * VZ == n2) *cells = n2;
+    return best;
+}
+
 // The split of a march over `count` meshes of shape n, or lz = 0 where a row does not hold a tile.
 template <typename A> static MarchSplit march_split(const int n[3], int count) {
     MarchSplit sp = {};
     constexpr int VZ = MarchVZ<A>::value;
-    // lanes a row: the power of two that computes the least, each segment's halo counted
-    int least = 0;
-    for (int lz = 32; lz >= 4; lz >>= 1) {
-        const int tz = lz * VZ, cells = (n[2] + tz - 1) / tz * (tz + 2 * VZ);
-        if (tz <= n[2] && (sp.lz == 0 || cells < least)) sp.lz = lz, least = cells;
-    }
+    int cells;
+    sp.lz = march_lanes<A>(n[2], &cells);
     if (sp.lz == 0) return sp;
     const int tz = sp.lz * VZ, rows = MARCH_THREADS / sp.lz;
     sp.zsegs = (n[2] + tz - 1) / tz;
     sp.ytiles = (n[1] + rows - 1) / rows;
     // the slab length whose waves of blocks (two a SM) take the fewest plane steps; a block's two outer planes and the
-    // fill of its pipeline count MARCH_FILL
+    // fill of its pipeline count MARCH_FILL.  Each length once, from the longest down: 2 sqrt(n0) of them, on every launch.
     const int64_t slots = 2 * (int64_t)device_sm_count(), tiles = (int64_t)sp.zsegs * sp.ytiles * count;
     int64_t best = 0;
-    for (int ns = 1; ns <= n[0]; ns++) {
-        const int slab = (n[0] + ns - 1) / ns, real = (n[0] + slab - 1) / slab;
+    for (int slab = n[0];;) {
+        const int real = (n[0] + slab - 1) / slab;
         const int64_t cost = (tiles * real + slots - 1) / slots * (slab + MARCH_FILL);
         if (best == 0 || cost < best) best = cost, sp.slab = slab, sp.nslab = real;
+        if (slab == 1) break;
+        const int more = (n[0] + slab - 2) / (slab - 1);       // the fewest slabs shorter than this one
+        slab = (n[0] + more - 1) / more;
     }
     return sp;
 }

@@ -863,10 +863,20 @@ static bool quad_ok(const int n[3], const void* a, const void* b, const void* c)
 // and a row holds a tile.
 // Below MARCH_MIN_BYTES of v the quad kernels are as fast (64^3 FP32, 1 MB: 3.2 against 3.7 us, the march's pipeline
 // fill; 96^3 FP32, 3.5 MB: 6.0 against 4.7 us; 64^3 FP64, 2 MB: 4.2 against 4.0 us).
-constexpr int64_t MARCH_MIN_BYTES = 3 << 19;
-template <typename A> static bool march_ok(const Stencil<A>& s, int count) {
-    return mg_mode(s) <= MG_LOCAL && s.n[2] >= 4 * MarchVZ<A>::value && (int64_t)s.n[0] * count <= 65535 &&
-           (int64_t)s.n[0] * s.n[1] * s.n[2] * count * (int64_t)sizeof(A) >= MARCH_MIN_BYTES;
+// FP32 rows that segments cover badly (march_lanes computes more than 29 / 20 of their cells): sweeps need MARCH_WIDE_BYTES
+// and go to the quad kernels beyond 9 / 5, residuals (a write-only output more to gain) beyond 2.  A sweep, quad kernel and
+// march: 128 x 128 x 44 (1.64) 5.0 and 5.5 us, 80^3 (1.5) 4.3 and 4.6, 300 x 200 x 52 (1.54, 12 MB) 14.1 and 13.2, 252 x 100
+// x 36 (2.0) 7.1 and 8.2, 1000 x 200 x 20 (2.4) 22.6 and 26.5; a residual of 80^3 5.9 and 4.7, 1000 x 200 x 20 27.5 and
+// 30.7.  In FP64 the march is ahead wherever a row holds a tile (1000 x 200 x 20: 60 and 44 us).
+constexpr int64_t MARCH_MIN_BYTES = 3 << 19, MARCH_WIDE_BYTES = 4 << 20;
+template <typename A> static bool march_ok(const Stencil<A>& s, int count, int op) {
+    int cells;
+    if (mg_mode(s) > MG_LOCAL || march_lanes<A>(s.n[2], &cells) == 0 || (int64_t)s.n[0] * count > 65535) return false;
+    const int64_t bytes = (int64_t)s.n[0] * s.n[1] * s.n[2] * count * (int64_t)sizeof(A);
+    if (bytes < MARCH_MIN_BYTES) return false;
+    if (sizeof(A) == 8 || 20 * cells <= 29 * s.n[2]) return true;
+    if (op == OP_RESIDUAL) return cells <= 2 * s.n[2];
+    return 5 * cells <= 9 * s.n[2] && bytes >= MARCH_WIDE_BYTES;
 }
 
 template <typename A, typename OT, int OP>
@@ -1022,7 +1032,7 @@ template <typename T> struct MGRunner {
             const bool z0 = zero_first && it == 0;
             double* a = it + 1 == niter ? acc : nullptr;
             const double bytes = (double)N * (sizeof(T) * (z0 ? 1 : 2) + (a != nullptr ? 16 : sizeof(T)));
-            if (quad && !z0 && march_ok(s, count)) {
+            if (quad && !z0 && march_ok(s, count, OP_JACOBI)) {
                 if (a != nullptr)
                     PRC_LAUNCH_B("mg_jacobi_add", st, bytes,
                                  (launch_march<T, T, OP_JACOBI_ADD>(v, f, tmp, a, s, (T)P.damping, count, st)));
@@ -1115,7 +1125,7 @@ template <typename T> struct MGRunner {
             Stencil<T> s = stencil(l);
             const int64_t N = L[l].size() * count;
             const Grid3 g = grid3(L[l].n, count);
-            if (quad_ok(L[l].n, v, f, B[l].r) && march_ok(s, count)) {
+            if (quad_ok(L[l].n, v, f, B[l].r) && march_ok(s, count, OP_RESIDUAL)) {
                 PRC_LAUNCH_B("mg_residual", st, 3.0 * N * sizeof(T),
                              (launch_march<T, T, OP_RESIDUAL>(v, f, B[l].r, nullptr, s, (T)0, count, st)));
             } else if (quad_ok(L[l].n, v, f, B[l].r)) {
@@ -1300,7 +1310,7 @@ int solve_mixed(const int32_t nmesh[3], const Params& P, void* ws, cudaStream_t 
                                                    P.has_los ? P.los : nullptr);
         for (int it = 0; it < P.vn; it++) {
             // defect in FP64 (stored FP32 as the inner V-cycle's right-hand side)
-            if (quad_ok(m.L[l].n, m.v64[l], m.f64[l], R.B[l].f) && march_ok(s64, count)) {
+            if (quad_ok(m.L[l].n, m.v64[l], m.f64[l], R.B[l].f) && march_ok(s64, count, OP_RESIDUAL)) {
                 PRC_LAUNCH_B("mg_residual_fp64", st, 20.0 * N,
                              (launch_march<double, float, OP_RESIDUAL>(m.v64[l], m.f64[l], R.B[l].f, nullptr,
                                                                                s64, 0., count, st)));
@@ -1599,7 +1609,7 @@ prc_status_t prc_multigrid_f64(const double* delta, double* phi, const int32_t n
         int n[3] = {nmesh[0], nmesh[1], nmesh[2]};                                                                   \
         Stencil<T> s = make_stencil<T>(n, boxsize, boxcenter, beta, los);                                            \
         const double bytes = 3.0 * sizeof(T) * n[0] * n[1] * n[2];                                                   \
-        if (quad_ok(n, v, f, r) && march_ok(s, 1))                                                             \
+        if (quad_ok(n, v, f, r) && march_ok(s, 1, OP_RESIDUAL))                                                             \
             PRC_LAUNCH_B("mg_residual", (cudaStream_t)stream, bytes,                                                 \
                          (launch_march<T, T, OP_RESIDUAL>(v, f, r, nullptr, s, (T)0, 1, (cudaStream_t)stream)));   \
         else if (quad_ok(n, v, f, r))                                                                                     \
