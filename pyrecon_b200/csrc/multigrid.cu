@@ -916,10 +916,16 @@ static cudaError_t launch_reduce(const T* fine, T* coarse, const int nf[3], int 
 template <typename T, bool ADD>
 static cudaError_t launch_prolong(const T* coarse, T* fine, const int nc[3], int count, cudaStream_t st) {
     const Dims d = {{nc[0], nc[1], nc[2]}};
-    const int half[3] = {nc[0], nc[1], nc[2] / 2};
-    const bool pair = nc[2] % 2 == 0 && (((uintptr_t)fine | (uintptr_t)coarse) & 15) == 0;
-    const Grid3 g = grid3(pair ? half : nc, count);
-    return launch_pdl(pair ? prolong_pair<T, ADD> : prolong_kernel<T, T, T, ADD>, g.grid, g.block, 0, st, coarse, fine, d);
+    // an FP64 mesh that is only written: one coarse cell a thread is faster (256^3 27 us, two 39)
+    if constexpr (ADD || sizeof(T) == 4) {
+        if (nc[2] % 2 == 0 && (((uintptr_t)fine | (uintptr_t)coarse) & 15) == 0) {
+            const int half[3] = {nc[0], nc[1], nc[2] / 2};
+            const Grid3 g = grid3(half, count);
+            return launch_pdl(prolong_pair<T, ADD>, g.grid, g.block, 0, st, coarse, fine, d);
+        }
+    }
+    const Grid3 g = grid3(nc, count);
+    return launch_pdl(prolong_kernel<T, T, T, ADD>, g.grid, g.block, 0, st, coarse, fine, d);
 }
 
 // Tile of the temporal-blocked sweeps: TB_TY rows x 4 TB_TQ cells.
