@@ -1403,7 +1403,8 @@ int paint_run(double* mesh, double* colsums, const BoxGeom& g, const P* pos, con
     PRC_LAUNCH_B("paint_columns", st, 8.0 * n + 4.0 * ncol, column_starts<<<particle_grid(n + 1), 256, 0, st>>>(keys, n, g.n[2], ncol, ws.col_start, flags));
     PRC_CHECK_LAUNCH();
     size_t smem = (size_t)PULL_WARPS * g.n[2] * sizeof(double);
-    if (smem > 48 * 1024) cudaFuncSetAttribute(paint_pull<F>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    // the same bound for every mesh: another thread's shorter rows must not lower it before this launch
+    if (smem > 48 * 1024) cudaFuncSetAttribute(paint_pull<F>, cudaFuncAttributeMaxDynamicSharedMemorySize, MAX_BLOCK_SMEM);
     int64_t blocks = (ncol + PULL_WARPS - 1) / PULL_WARPS;
     int grid = (int)std::min<int64_t>(blocks, (int64_t)device_sm_count() * 16);
     Dims dims = {{g.n[0], g.n[1], g.n[2]}};

@@ -1032,6 +1032,12 @@ static bool spectrum_map(CUtensorMap* m, const void* base, const Plan3& p, size_
                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// The mixed-radix kernels' shared memory differs from launch to launch, so every launch sets the same bound: with its own
+// size, another thread's shorter line could lower the bound between this call and the launch, which then fails.
+template <typename K> static void any_shared_memory(K kern) {
+    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, MAX_BLOCK_SMEM);
+}
+
 // Persistent grid: as many CTAs as fit on the device at once (occupancy of this launch), at most one per tile.
 template <typename K> static int resident_grid(K kern, int threads, size_t smem, int64_t ntiles) {
     // occupancy of (kernel, device, threads, shared memory), looked up once: a mixed-radix kernel's shared memory differs
@@ -1376,7 +1382,7 @@ template <typename T> struct FFTLaunch {
     static int strided_blocks(int n) {
         size_t smem;
         strided_lines(n, &smem);
-        cudaFuncSetAttribute(fft_strided<T, -1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        any_shared_memory(fft_strided<T, -1>);
         return resident_grid(fft_strided<T, -1>, FFT_THREADS, smem, INT_MAX) / device_sm_count();
     }
 
@@ -1403,7 +1409,7 @@ template <typename T> struct FFTLaunch {
             ri.p[i] = in[i];
             so.p[i] = out[i];
         }
-        cudaFuncSetAttribute(fft_z_r2c<T, TIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        any_shared_memory(fft_z_r2c<T, TIN>);
         int64_t rows = (int64_t)p.dims.n[0] * p.dims.n[1];
         int64_t ntiles = ((rows + B - 1) / B) * nb;
         PRC_LAUNCH_B("fft_z_r2c", st, (double)nb * rows * (p.dims.n[2] * sizeof(TIN) + p.nh * CS), fft_z_r2c<T, TIN><<<resident_grid(fft_z_r2c<T, TIN>, FFT_THREADS, smem, ntiles), FFT_THREADS, smem, st>>>(ri, so, nb, p.dims, p.pitch, p.rz, B));
@@ -1456,7 +1462,7 @@ template <typename T> struct FFTLaunch {
         const int B = strided_lines(s.n, &smem);
         Specs<C> sp;
         for (int i = 0; i < nb; i++) sp.p[i] = data[i];
-        cudaFuncSetAttribute(fft_strided<T, DIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        any_shared_memory(fft_strided<T, DIR>);
         int64_t ntiles = (int64_t)s.outer * ((nh + B - 1) / B) * nb;
         PRC_LAUNCH_B((DIR < 0 ? (axis == 1 ? "fft_y_fwd" : "fft_x_fwd") : (axis == 1 ? "fft_y_inv" : "fft_x_inv")), st, 2.0 * nb * spectrum_values(p) * CS, fft_strided<T, DIR><<<resident_grid(fft_strided<T, DIR>, FFT_THREADS, smem, ntiles), FFT_THREADS, smem, st>>>(sp, nb, s, axis == 1 ? p.ry : p.rx, B));
         PRC_CHECK_LAUNCH();
@@ -1482,7 +1488,7 @@ template <typename T> struct FFTLaunch {
         Specs<C> si, so;
         for (int i = 0; i < nin; i++) si.p[i] = in[i];
         for (int i = 0; i < nin * op.nper; i++) so.p[i] = out[i];
-        cudaFuncSetAttribute(fft_x_fused<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        any_shared_memory(fft_x_fused<T>);
         int64_t ntiles = (int64_t)p.dims.n[1] * ((p.nh + B - 1) / B) * nin;
         PRC_LAUNCH_B("fft_x_kspace", st, (double)nin * (1 + op.nper) * spectrum_values(p) * CS, fft_x_fused<T><<<resident_grid(fft_x_fused<T>, FFT_THREADS, smem, ntiles), FFT_THREADS, smem, st>>>(si, nin, so, p.dims, p.pitch, p.rx, B, op));
         PRC_CHECK_LAUNCH();
@@ -1528,7 +1534,7 @@ template <typename T> struct FFTLaunch {
         const size_t smem = need(B);
         Specs<C> si;
         for (int i = 0; i < nin; i++) si.p[i] = in[i];
-        cudaFuncSetAttribute(fft_z_c2r<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        any_shared_memory(fft_z_c2r<T>);
         int64_t rows = (int64_t)p.dims.n[0] * p.dims.n[1];
         int64_t ntiles = (rows + B - 1) / B;
         PRC_LAUNCH_B("fft_z_c2r", st, (double)nin * rows * nh * CS + (double)rows * p.dims.n[2] * sizeof(T) * (e.type == EPI_STORE ? nin : (e.delta ? 2 : 1)), fft_z_c2r<T><<<resident_grid(fft_z_c2r<T>, FFT_THREADS, smem, ntiles), FFT_THREADS, smem, st>>>(si, nin, p.dims, p.pitch, p.rz, B, e));
