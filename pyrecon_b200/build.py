@@ -33,9 +33,10 @@ FLAGS = ['-O3', '-std=c++17', '-lineinfo', '-Xcompiler', '-fPIC', '-Xcompiler', 
 
 
 # name -> (source rebuilt, extra nvcc flags).  'nopp': every TMA-fed FFT pass with two barriers per
-# shared-memory exchange instead of the ping-pong buffers (same arithmetic, same order).
+# shared-memory exchange instead of the ping-pong buffers, one column a thread (the same bits in FP32;
+# in FP64 the compiler fuses a k-space pass's multipliers differently).
 VARIANTS = {
-    'nopp': ('fft.cu', ['-DPRC_STRIDED_PP=0', '-DPRC_KSPACE_PP=0', '-DPRC_HESS_PP=0', '-DPRC_C2R_PP=0']),
+    'nopp': ('fft.cu', ['-DPRC_DUO=0', '-DPRC_STRIDED_PP=0', '-DPRC_KSPACE_PP=0', '-DPRC_HESS_PP=0', '-DPRC_C2R_PP=0']),
     # every radix-8 twiddle read from the pass table (7 loads per butterfly instead of 3 and 4 products)
     'twload': ('fft.cu', ['-DPRC_TW_RECUR=0']),
     # the z passes' row transforms with block barriers instead of warp barriers (same arithmetic, same order)

@@ -1104,6 +1104,11 @@ template <typename T, int N> struct StridedTmaCfg {
     static_assert(SMEM <= 227 * 1024, "a strided tile's stages fit on an SM");
 };
 
+// 0: one column a thread everywhere (the library variant that the tests compare with).
+#ifndef PRC_DUO
+#define PRC_DUO 1
+#endif
+
 // Pairs of columns a tile and blocks an SM of the FP32 passes on pairs of columns (fft_duo.cuh): about 16 warps an SM
 // (128 registers a thread).  Strided tiles have 128-byte rows where they fit; the k-space and Hessian passes 64-byte rows,
 // so that several blocks share an SM and a small mesh has tiles for all of them (k-space launch at 256: 0.100 ms against
@@ -1115,7 +1120,7 @@ template <typename T, int N> struct StridedTmaCfg {
 // SM differs) of the four operators below.  Lines of 3 2^k points, 1024-point k-space lines and the one-output iteration
 // along a fixed line of sight round elsewhere in their chains of products and sums, and keep one column a thread.
 template <int N> struct DuoCfg {
-    static constexpr bool OK = N >= 64 && N % 3 != 0, K_OK = OK && N <= 512;
+    static constexpr bool OK = PRC_DUO && N >= 64 && N % 3 != 0, K_OK = OK && N <= 512;
     static constexpr int KBP = 4, SBP = N >= 1024 ? 4 : 8, S = 2;
     static constexpr int KTHREADS = N / 8 * KBP, STHREADS = N / 8 * SBP;
     static constexpr size_t KSMEM = fast::KSpaceDuoSmem<N, KBP>::BYTES, SSMEM = fast::StridedDuoSmem<N, SBP, S>::BYTES;
