@@ -288,6 +288,10 @@ PRC_API int prc_debug_wait_timeout(int64_t limit_ns, int* out, void* stream);
  * runs out, of `stages` stages: all that may still be in flight (host arithmetic, the kernels' own function). */
 PRC_API int prc_debug_units_in_flight(int64_t unit, int stages);
 
+/* out[2 q] = q / divisor, out[2 q + 1] = q mod divisor (device) for q < count <= 65536, 1 <= divisor <= 2048, by the
+ * multiplication that the mixed-radix FFT passes index with. */
+PRC_API int prc_debug_quotients(int32_t divisor, int32_t count, int32_t* out, void* stream);
+
 /* Blocks an SM that the mixed-radix strided pass over lines of n points (2 <= n <= 2048) is launched with on the
  * current device (0 on a bad argument; nothing is launched). */
 PRC_API int prc_debug_fft_strided_blocks(int32_t n, int mesh_bytes);

@@ -42,6 +42,7 @@ _SIGNATURES = {
     'prc_device_fault_flags': (ctypes.c_uint, [c_int]),
     'prc_debug_wait_timeout': (c_int, [c_i64, _p, _p]),
     'prc_debug_units_in_flight': (c_int, [c_i64, c_int]),
+    'prc_debug_quotients': (c_int, [ctypes.c_int32, ctypes.c_int32, _p, _p]),
     'prc_debug_fft_strided_blocks': (c_int, [ctypes.c_int32, c_int]),
     'prc_tune_set': (c_int, [ctypes.c_char_p, c_int, c_int]),
     'prc_tune_get': (c_int, [ctypes.c_char_p, c_int, c_int]),

@@ -413,7 +413,8 @@ struct Strided {
     int ncols;      // columns (z extent nh)
 };
 
-// The first pass reads a tile and the last one writes it directly (B columns of a row are 64 to 256 contiguous bytes).
+// The first pass reads a tile and the last one writes it directly (B columns of a row are contiguous: 64 to 256
+// bytes at 8 or 16 columns, fewer on long lines, where choose_B takes down to one column).
 template <typename C> struct TileIn {
     const C* g;
     int64_t ls;
@@ -767,6 +768,16 @@ __global__ void debug_wait_timeout(uint64_t limit_ns, uint32_t bytes, int* out) 
         out[0] = done ? 0 : 1;
         tma::barrier_inval(&bar);
     }
+}
+
+// FastDiv's quotients and remainders of 0 .. count - 1.
+__global__ void debug_quotients(int divisor, int count, int* out) {
+    const int q = blockIdx.x * blockDim.x + threadIdx.x;
+    const FastDiv by(divisor);
+    if (q >= count) return;
+    const int quotient = by.div(q);
+    out[2 * q] = quotient;
+    out[2 * q + 1] = by.mod(q, quotient);
 }
 
 #include "fft_fast.cuh"
@@ -1902,6 +1913,14 @@ static bool geom_ok(const int32_t* nmesh, const double* boxsize) {
 }
 
 extern "C" {
+
+int prc_debug_quotients(int32_t divisor, int32_t count, int32_t* out, void* stream) {
+    if (!out || divisor < 1 || divisor > MAX_FFT_N || count < 1 || count > 1 << 16) return PRC_ERR_ARG;
+    cudaStream_t st = (cudaStream_t)stream;
+    PRC_LAUNCH("debug_quotients", st, debug_quotients<<<(count + 255) / 256, 256, 0, st>>>(divisor, count, out));
+    PRC_CHECK_LAUNCH();
+    return PRC_OK;
+}
 
 unsigned int prc_device_fault_flags(int reset) {
     unsigned int v = 0;
