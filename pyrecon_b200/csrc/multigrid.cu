@@ -24,6 +24,7 @@
 #include <mutex>
 #include <stdlib.h>
 #include <string>
+#include <tuple>
 #include <vector>
 
 namespace prc {
@@ -258,7 +259,8 @@ __device__ __forceinline__ void quad_terms(const QuadCols<T>& Q, const OpCoef<T>
 // U, W, q and P of the axis modes, which leave out terms that are exact zeros, and the damped-Jacobi values from them.  The
 // expressions are left to the compiler, for all four cells before the divisions: in pairs of cells, spelled out as op_terms,
 // they took 40 registers instead of 32 in the FP32 sweep and 70 instead of 64 in the FP64 one (a sweep at 256^3: FP32 33.8 us
-// and 37.3 in pairs, FP64 along y 78 and 95).
+// and 37.3 in pairs, FP64 along y 78 and 95; one cell at a time, spelled out, 38.7 and 85).  They come out as vcycle_coarse
+// spells them (the tests compare the bits).
 template <int MODE, typename T>
 __device__ __forceinline__ void axis_terms(const QuadCols<T>& Q, const Stencil<T>& s, T (&U)[4], T (&W)[4], T (&qq)[4],
                                            T (&P)[4]) {
@@ -282,11 +284,13 @@ __device__ __forceinline__ void axis_terms(const QuadCols<T>& Q, const Stencil<T
 template <typename T>
 __device__ __forceinline__ void axis_zero_terms(const Stencil<T>& s, T (&U)[4], T (&W)[4], T (&qq)[4], T (&P)[4], T (&vc)[4]) {
     const T p0 = s.losh[0], p1 = s.losh[1], p2 = s.losh[2];
+    const T s0 = p0 * p0, s1 = p1 * p1;
+    const T q01 = s.h2[0] * s0 + s.h2[1] * s1, P01 = s0 + s1;
 #pragma unroll
     for (int k = 0; k < 4; k++) {
         const T s2 = p2 * p2;
-        qq[k] = s.h2[0] * p0 * p0 + s.h2[1] * p1 * p1 + s.h2[2] * s2;
-        P[k] = p0 * p0 + p1 * p1 + s2;
+        qq[k] = q01 + s.h2[2] * s2;
+        P[k] = P01 + s2;
         U[k] = W[k] = vc[k] = (T)0;
     }
 }
@@ -403,7 +407,7 @@ __global__ void __launch_bounds__(256) jacobi_sweep4(const T* __restrict__ v, co
 // row and one quad on each side into a ring of three planes in shared memory, then the second sweep at
 // plane x - 1 over the tile from the ring's planes x - 2 .. x.  v and f are read from DRAM once and the
 // result written once per two sweeps (the halo of the first sweep is recomputed by the neighbouring
-// tiles).  Every quad goes through quad_compute / quad_blend, the arithmetic of jacobi_sweep4, so two
+// tiles).  Every quad goes through quad_jacobi, the arithmetic of jacobi_sweep4, so two
 // sweeps here equal two jacobi_sweep4 launches bit for bit.  Periodic in every axis: staged rows and
 // 4-cell chunks wrap (n2 % 4 == 0 keeps every chunk contiguous and aligned).
 template <typename T, int TY, int TQ> struct TbShape {
@@ -1061,8 +1065,39 @@ template <typename T> struct MGRunner {
         return PRC_OK;
     }
 
+    // Clusters of cl blocks of a coarse kernel that run on the device at once, looked up once for each shared-memory size.
+    template <typename K> static int clusters_at_once(K kernel, int cl, size_t smem) {
+        typedef std::tuple<const void*, int, int, size_t> Key;
+        static std::mutex mu;
+        static std::map<Key, int> known;
+        int dev = 0;
+        cudaGetDevice(&dev);
+        std::lock_guard<std::mutex> lock(mu);
+        const Key key((const void*)kernel, dev, cl, smem);
+        const auto it = known.find(key);
+        if (it != known.end()) return it->second;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(cl);
+        cfg.blockDim = dim3(MG_COARSE_THREADS);
+        cfg.dynamicSmemBytes = smem;
+        cudaLaunchAttribute attr = {};
+        attr.id = cudaLaunchAttributeClusterDimension;
+        attr.val.clusterDim.x = cl;
+        attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+        cfg.attrs = &attr;
+        cfg.numAttrs = 1;
+        int n = 0;
+        if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) {
+            cudaGetLastError();
+            n = 0;
+        }
+        return known[key] = n;
+    }
+
     // The V-cycle from level l down as one vcycle_coarse launch, when level l has at most "mg_small_cells"
     // cells (run-time knob, key 0; 0 runs every step as its own kernel) and its levels fit in shared memory.
+    // Of cubes the largest it takes is 20^3: a block has threads for 1024 pairs of cells of its top level, and of 24^3, dealt
+    // as twice the planes of 12^3, one would hold four planes, 1152 pairs.
     int coarse_vcycle(int l, T* v, const T* f, bool v_zero, bool* done) {
         *done = false;
         const int limit = tune_get("mg_small_cells", 0, MG_COARSE_DEFAULT_CELLS);
@@ -1100,6 +1135,10 @@ template <typename T> struct MGRunner {
         const auto kernel = c.s[0].local ? vcycle_coarse<T, true> : vcycle_coarse<T, false>;
         if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MG_COARSE_MAX_SMEM) != cudaSuccess)
             return PRC_ERR_CUDA;
+        // A batch whose clusters do not run at once takes the dealt levels by launches (same bits) and comes back with the
+        // levels of one block: whole solves by clusters and so, 14 of 32^3 FP32 0.89 and 1.06 ms, 16 1.18 and 1.06, 32 of
+        // 40^3 FP64 along z 3.43 and 2.57, 16 of 64^3 FP64 4.84 and 4.62.
+        if (c.ndist > 0 && clusters_at_once(kernel, cl, smem) < count) return PRC_OK;
         PRC_LAUNCH_B("mg_vcycle_coarse", st, (double)L[l].size() * count * sizeof(T) * (v_zero ? 2 : 3),
                      launch_cluster_pdl(kernel, dim3(cl * count), dim3(MG_COARSE_THREADS), cl, smem, st, f, v, c));
         PRC_CHECK_LAUNCH();
