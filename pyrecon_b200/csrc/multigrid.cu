@@ -872,10 +872,15 @@ static bool quad_ok(const int n[3], const void* a, const void* b, const void* c)
 // march: 128 x 128 x 44 (1.64) 5.0 and 5.5 us, 80^3 (1.5) 4.3 and 4.6, 300 x 200 x 52 (1.54, 12 MB) 14.1 and 13.2, 252 x 100
 // x 36 (2.0) 7.1 and 8.2, 1000 x 200 x 20 (2.4) 22.6 and 26.5; a residual of 80^3 5.9 and 4.7, 1000 x 200 x 20 27.5 and
 // 30.7.  In FP64 the march is ahead wherever a row holds a tile (1000 x 200 x 20: 60 and 44 us).
+// Where half the rows of the tiles lie past the mesh, or a third of 32 and more, the quad kernels stay: solves in FP64 by them
+// and marched, 640 x 24 x 24 (24 rows of 64) 1.78 and 2.03 ms, 2000 x 20 x 16 (20 of 32) 1.45 and 1.54.
 constexpr int64_t MARCH_MIN_BYTES = 3 << 19, MARCH_WIDE_BYTES = 4 << 20;
 template <typename A> static bool march_ok(const Stencil<A>& s, int count, int op) {
     int cells;
-    if (mg_mode(s) > MG_LOCAL || march_lanes<A>(s.n[2], &cells) == 0 || (int64_t)s.n[0] * count > 65535) return false;
+    const int lz = march_lanes<A>(s.n[2], &cells);
+    if (mg_mode(s) > MG_LOCAL || lz == 0 || (int64_t)s.n[0] * count > 65535) return false;
+    const int rows = MARCH_THREADS / lz;
+    if (2 * ((s.n[1] + rows - 1) / rows * rows) >= (rows >= 32 ? 3 : 4) * s.n[1]) return false;
     const int64_t bytes = (int64_t)s.n[0] * s.n[1] * s.n[2] * count * (int64_t)sizeof(A);
     if (bytes < MARCH_MIN_BYTES) return false;
     if (sizeof(A) == 8 || 20 * cells <= 29 * s.n[2]) return true;
