@@ -322,6 +322,35 @@ __device__ __forceinline__ void quad_jacobi(const QuadCols<T>& Q, const OpCoef<T
     }
 }
 
+// The sums of a quad's cells 2 j, 2 j + 1 in a pair, FP32 meshes below MARCH_MIN_BYTES: fewer instructions, and there no
+// sweep waits on memory bandwidth (60 sweeps and their residuals at 100 x 60 x 44 in a solve of 1.00 ms: 0.94 in pairs).
+// The same operations: the same bits.
+template <bool LOCAL, typename T, typename P2 = typename Pair<T>::T>
+__device__ __forceinline__ void quad_pair_terms(const QuadCols<T>& Q, const OpCoef<T>& k, const XYCoef<T>& c, int z0, int i,
+                                                P2& U, P2& W, P2& q, P2& PP) {
+    typedef Pair<T> P;
+    auto two = [](const T* a) { return P::make(a[0], a[1]); };
+    const P2 p2 = P::make(z_p2<LOCAL>(k, z0 + i), z_p2<LOCAL>(k, z0 + i + 1)), s2 = P::mul(p2, p2);
+    const P2 exy = P::sub(P::add(two(Q.PP + i), two(Q.MM + i)), P::add(two(Q.MP + i), two(Q.PM + i)));
+    const P2 exz = P::sub(P::add(two(Q.XP + i + 2), two(Q.XM + i)), P::add(two(Q.XM + i + 2), two(Q.XP + i)));
+    const P2 eyz = P::sub(P::add(two(Q.YP + i + 2), two(Q.YM + i)), P::add(two(Q.YM + i + 2), two(Q.YP + i)));
+    op_terms<LOCAL, P>(k, c, p2, s2, two(Q.XP + i + 1), two(Q.XM + i + 1), two(Q.YP + i + 1), two(Q.YM + i + 1),
+                       two(Q.c + i + 2), two(Q.c + i), exy, exz, eyz, U, W, q, PP);
+}
+template <bool LOCAL, typename T>
+__device__ __forceinline__ void quad_pairs_jacobi(const QuadCols<T>& Q, const OpCoef<T>& k, T w, int x, int y, int z0,
+                                                  const T (&f)[4], T (&o)[4]) {
+    typedef Pair<T> P;
+    const XYCoef<T> c = xy_coef<LOCAL>(k, x, y);
+#pragma unroll
+    for (int i = 0; i < 4; i += 2) {
+        typename P::T U, W, q, PP;
+        quad_pair_terms<LOCAL>(Q, k, c, z0, i, U, W, q, PP);
+        const typename P::T r = op_jacobi<P>(k, P::make(f[i], f[i + 1]), P::make(Q.c[i + 1], Q.c[i + 2]), U, W, q, PP, w);
+        o[i] = r.x, o[i + 1] = r.y;
+    }
+}
+
 // The same where v is identically zero (the first sweep of a V-cycle started from zero): w q f / den, with q and P
 // summed in their own order (local: h_0^2 p_0^2 and h_1^2 p_1^2 as (h^2 p) p).
 template <bool LOCAL, typename T>
@@ -355,8 +384,8 @@ template <typename T> __device__ __forceinline__ void store4(T* p, const T (&o)[
 
 // Damped-Jacobi sweep of four cells per thread: the axis modes, the 19-point ones where march_ok leaves them here (short
 // rows, small meshes), and (zero_v) every sweep from an identically zero v.
-// ADD: the sweep's result is added to acc instead of being stored (OP_JACOBI_ADD).
-template <typename T, int MODE, bool ADD>
+// ADD: the sweep's result is added to acc instead of being stored (OP_JACOBI_ADD).  PAIRS: 19-point, by quad_pair_terms.
+template <typename T, int MODE, bool ADD, bool PAIRS>
 __global__ void __launch_bounds__(256) jacobi_sweep4(const T* __restrict__ v, const T* __restrict__ f,
                                                      T* __restrict__ vout, double* __restrict__ acc, Stencil<T> s, T w,
                                                      int zero_v) {
@@ -384,7 +413,8 @@ __global__ void __launch_bounds__(256) jacobi_sweep4(const T* __restrict__ v, co
     } else {
         QuadCols<T> Q;
         quad_load<MODE>(v, s, q, Q);
-        quad_jacobi<MODE == MG_LOCAL>(Q, op_coef<MODE == MG_LOCAL>(s), w, q.x, q.y, q.z0, fv, o);
+        if constexpr (PAIRS) quad_pairs_jacobi<MODE == MG_LOCAL>(Q, op_coef<MODE == MG_LOCAL>(s), w, q.x, q.y, q.z0, fv, o);
+        else quad_jacobi<MODE == MG_LOCAL>(Q, op_coef<MODE == MG_LOCAL>(s), w, q.x, q.y, q.z0, fv, o);
     }
     if constexpr (ADD) {
         double* a = acc + bo + q.c + q.z0;
@@ -618,13 +648,14 @@ __global__ void __launch_bounds__(256) residual_kernel(const V* __restrict__ v, 
 }
 
 // The quad kernels' instance for an operator form (mg_mode).
-template <typename T, bool ADD> static decltype(&jacobi_sweep4<T, MG_GLOBAL, ADD>) sweep4_kernel(int mode) {
+template <typename T, bool ADD> static decltype(&jacobi_sweep4<T, MG_GLOBAL, ADD, false>) sweep4_kernel(int mode, bool small) {
+    constexpr bool PAIRS = sizeof(T) == 4;
     switch (mode) {
-    case MG_LOCAL: return jacobi_sweep4<T, MG_LOCAL, ADD>;
-    case MG_AXIS0: return jacobi_sweep4<T, MG_AXIS0, ADD>;
-    case MG_AXIS1: return jacobi_sweep4<T, MG_AXIS1, ADD>;
-    case MG_AXIS2: return jacobi_sweep4<T, MG_AXIS2, ADD>;
-    default: return jacobi_sweep4<T, MG_GLOBAL, ADD>;
+    case MG_LOCAL: return small ? jacobi_sweep4<T, MG_LOCAL, ADD, PAIRS> : jacobi_sweep4<T, MG_LOCAL, ADD, false>;
+    case MG_AXIS0: return jacobi_sweep4<T, MG_AXIS0, ADD, false>;
+    case MG_AXIS1: return jacobi_sweep4<T, MG_AXIS1, ADD, false>;
+    case MG_AXIS2: return jacobi_sweep4<T, MG_AXIS2, ADD, false>;
+    default: return small ? jacobi_sweep4<T, MG_GLOBAL, ADD, PAIRS> : jacobi_sweep4<T, MG_GLOBAL, ADD, false>;
     }
 }
 template <typename A, typename R> static decltype(&residual_kernel4<A, R, MG_GLOBAL>) residual4_kernel(int mode) {
@@ -1026,6 +1057,7 @@ template <typename T> struct MGRunner {
         if (niter == 0 && zero_first && cudaMemsetAsync(v, 0, N * sizeof(T), st) != cudaSuccess) return PRC_ERR_CUDA;
         const bool quad = quad_ok(L[l].n, v, f, tmp);
         const Grid3 gq = grid3_quad(L[l].n, count);
+        const bool small = N * (int64_t)sizeof(T) < MARCH_MIN_BYTES;
         int it = 0;
         const int slab =
             quad ? tune_get(sizeof(T) == 4 ? "mg_jacobi" : "mg_jacobi_f64", L[l].n[0], mg_tb_default(L[l].n, sizeof(T)))
@@ -1056,7 +1088,7 @@ template <typename T> struct MGRunner {
                                  (launch_march<T, T, OP_JACOBI>(v, f, tmp, nullptr, s, (T)P.damping, count, st)));
             } else if (quad) {
                 PRC_LAUNCH_B(a != nullptr ? "mg_jacobi_add" : "mg_jacobi", st, bytes,
-                             launch_pdl(a != nullptr ? sweep4_kernel<T, true>(mg_mode(s)) : sweep4_kernel<T, false>(mg_mode(s)), gq.grid, gq.block, 0, st, v, f, tmp, a, s, (T)P.damping, z0));
+                             launch_pdl(a != nullptr ? sweep4_kernel<T, true>(mg_mode(s), small) : sweep4_kernel<T, false>(mg_mode(s), small), gq.grid, gq.block, 0, st, v, f, tmp, a, s, (T)P.damping, z0));
             } else {
                 PRC_LAUNCH_B("mg_jacobi", st, (double)N * sizeof(T) * (z0 ? 2 : 3),
                              launch_pdl(jacobi_sweep<T, T>, g.grid, g.block, 0, st, v, f, tmp, s, (T)P.damping, z0));
