@@ -1147,6 +1147,10 @@ template <typename T> struct MGRunner {
         const int slots = MG_COARSE_SLOTS * MG_COARSE_THREADS;
         while (c.ndist < nl && L[l + c.ndist].size() > MG_SINGLE_CELLS && L[l + c.ndist].n[2] % 4 == 0) c.ndist++;
         if (c.ndist < nl && L[l + c.ndist].size() > slots) return PRC_OK;
+        // a lone level has only its ten sweeps to save, and in FP64 or with the seven terms of an axis a launched sweep is
+        // short: solves by launches and in a cluster, 512 x 64 x 16 (128 x 16 x 4 the coarsest) FP64 1.26 and 1.30 ms, along
+        // y 0.93 and 1.00, 2000 x 20 x 16 FP32 along y 0.70 and 0.77; but 64 x 512 x 16 FP32 oblique 0.87 and 0.84
+        if (nl == 1 && c.ndist == 1 && (sizeof(T) == 8 || mg_mode(stencil(l)) >= MG_AXIS0)) return PRC_OK;
         c.base = c.ndist > 0 ? L[l + c.ndist - 1].n[0] : 0;
         int cl = 1;
         while (c.ndist > 0 && 2 * cl <= std::min(c.base, MG_COARSE_CLUSTER)) cl *= 2;
