@@ -21,6 +21,7 @@
 #include <algorithm>
 #include <map>
 #include <mutex>
+#include <type_traits>
 
 namespace prc {
 
@@ -894,20 +895,21 @@ __device__ __forceinline__ void cic_read3(const typename vec4_of<F>::type* __res
 
 // Finite-difference gradient CIC read (src/mesh.c:187-266): corners in the order
 // 000, 100, 010, 001, 110, 101, 011, 111; divided by 2 * boxsize / n in F.
-template <typename F>
+template <typename OFF, typename F>
 __device__ __forceinline__ void fd_read(const F* __restrict__ m, const Cic<F>& c, const int n[3], const F twocell[3],
                                         F out[3]) {
     // Along each axis the eight corners and their +-1 neighbours span four nodes, lo - 1, lo, hi, hi + 1
     // (periodic), indexed 0..3: corner c (0 or 1) sits at index c + 1, its neighbours at c and c + 2.  The
     // 32 distinct values are loaded once from precomputed plane, row and cell offsets; the arithmetic and
     // its order are those of the corner loop of src/mesh.c:187-266.
-    // 64-bit offsets: with 32-bit ones the compiler keeps fewer loads in flight, and particles in no order wait longer
-    // (4M FP64 ones on an FP64 mesh of 384^3: 1.19 ms, 1.08 with these; 512^3 1.63 and 1.49).
-    const int64_t sx = (int64_t)n[1] * n[2];
-    const int64_t X[4] = {wrap_dn(c.lo[0], n[0]) * sx, c.lo[0] * sx, c.hi[0] * sx, wrap_up(c.hi[0], n[0]) * sx};
-    const int64_t Y[4] = {(int64_t)wrap_dn(c.lo[1], n[1]) * n[2], (int64_t)c.lo[1] * n[2], (int64_t)c.hi[1] * n[2],
-                          (int64_t)wrap_up(c.hi[1], n[1]) * n[2]};
-    const int Z[4] = {wrap_dn(c.lo[2], n[2]), c.lo[2], c.hi[2], wrap_up(c.hi[2], n[2])};
+    // Offsets along x and y in OFF (a mesh has fewer than 2^32 cells, checked by the entry points).  With 32-bit ones the
+    // compiler keeps fewer loads in flight, and particles in no order wait longer (4M FP64 ones on an FP64 mesh of 384^3:
+    // 1.19 ms, 1.08 with 64-bit ones; 512^3 1.63 and 1.49); in cell order they are a little faster (FP32 64^3 0.169 and 0.163).
+    typedef typename std::conditional<sizeof(OFF) == 8, int, OFF>::type ZOFF;
+    const OFF sy = n[2], sx = (OFF)n[1] * sy;
+    const OFF X[4] = {wrap_dn(c.lo[0], n[0]) * sx, c.lo[0] * sx, c.hi[0] * sx, wrap_up(c.hi[0], n[0]) * sx};
+    const OFF Y[4] = {wrap_dn(c.lo[1], n[1]) * sy, c.lo[1] * sy, c.hi[1] * sy, wrap_up(c.hi[1], n[1]) * sy};
+    const ZOFF Z[4] = {(ZOFF)wrap_dn(c.lo[2], n[2]), (ZOFF)c.lo[2], (ZOFF)c.hi[2], (ZOFF)wrap_up(c.hi[2], n[2])};
     F xv[4][2][2], yv[2][4][2], zv[2][2][4];   // [axis index 0..3 along the derivative's axis][corner][corner]
 #pragma unroll
     for (int a = 0; a < 2; a++)
@@ -916,9 +918,9 @@ __device__ __forceinline__ void fd_read(const F* __restrict__ m, const Cic<F>& c
 #pragma unroll
             for (int e = 0; e < 4; e++) {
                 const bool core = e == 1 || e == 2;
-                xv[e][a][b] = __ldg(m + X[e] + Y[a + 1] + Z[b + 1]);
-                yv[a][e][b] = core ? F(0) : __ldg(m + X[a + 1] + Y[e] + Z[b + 1]);
-                zv[a][b][e] = core ? F(0) : __ldg(m + X[a + 1] + Y[b + 1] + Z[e]);
+                xv[e][a][b] = __ldg(m + (X[e] + Y[a + 1] + Z[b + 1]));
+                yv[a][e][b] = core ? F(0) : __ldg(m + (X[a + 1] + Y[e] + Z[b + 1]));
+                zv[a][b][e] = core ? F(0) : __ldg(m + (X[a + 1] + Y[b + 1] + Z[e]));
             }
         }
     // core nodes (indices 1, 2 on every axis) come from the x table
@@ -985,7 +987,7 @@ __global__ void __launch_bounds__(256) read_fd_kernel(const F* __restrict__ mesh
         int bad = 0;
         if (i < n) {
             F q[3] = {0, 0, 0}, s[3] = {(F)NAN, (F)NAN, (F)NAN};
-            if (particle_index<P, F>(pos, i, g, wrap, q, &bad)) fd_read(mesh, cic_setup(q, g.n), g.n, twocell, s);
+            if (particle_index<P, F>(pos, i, g, wrap, q, &bad)) fd_read<int64_t>(mesh, cic_setup(q, g.n), g.n, twocell, s);
 #pragma unroll
             for (int a = 0; a < 3; a++) out[3 * i + a] = (P)s[a];
         }
@@ -1010,14 +1012,15 @@ __global__ void __launch_bounds__(256) read_fd_kernel(const F* __restrict__ mesh
 // registers left one block on an SM, 12 % of its warps, waiting on memory; 128 threads at four blocks took the read-outs of
 // a nmesh-256 multigrid reconstruction (12M particles, FP64 from an FP64 potential, in cell order) from 1.03 to 0.75 ms,
 // 512 (25M) 2.32 to 1.87, against 0.79 and 2.01 with five blocks, 0.77 and 2.07 with six, 0.83 and 2.69 with eight.
-// Three blocks (FAR) where more warps only miss the caches more: all in FP32 (4M particles in no order, 128^3, four blocks
-// and three: 0.308 and 0.296 ms, 512^3 1.09 and 0.99; in cell order the same), and particles in no order on a mesh well
-// beyond the L2 (FP64 from FP64, 512^3 1.49 and 1.41, 384^3 1.08 and 1.01, but 64^3 0.344 and 0.357).
+// In no order three blocks (PHI_FAR) where more warps only miss the caches more: all in FP32 (4M particles, 128^3, four
+// blocks and three: 0.308 and 0.296 ms, 512^3 1.09 and 0.99), and on a mesh well beyond the L2 (FP64 from FP64, 512^3 1.49
+// and 1.41, 384^3 1.08 and 1.01, but 64^3 0.344 and 0.357).
+enum { PHI_NEAR = 0, PHI_FAR = 1, PHI_ORDERED = 2 };
 constexpr int PHI_THREADS = 128;
 constexpr double PHI_FAR_BYTES = 2e8;
 
-template <typename P, typename F, typename O, bool PHI, bool IL, bool FAR>
-__global__ void __launch_bounds__((PHI ? PHI_THREADS : 256), (PHI ? (FAR ? 3 : 4) : PRC_READ_MINB)) read_shifts_kernel(const F* __restrict__ m0, const F* __restrict__ m1,
+template <typename P, typename F, typename O, bool PHI, bool IL, int SHAPE>
+__global__ void __launch_bounds__((PHI ? PHI_THREADS : 256), (PHI ? (SHAPE == PHI_FAR ? 3 : 4) : PRC_READ_MINB)) read_shifts_kernel(const F* __restrict__ m0, const F* __restrict__ m1,
                                                           const F* __restrict__ m2, BoxGeom g, F tc0, F tc1, F tc2,
                                                           const P* __restrict__ pos, int64_t n, double f,
                                                           int global_los, double l0, double l1, double l2, int field,
@@ -1056,7 +1059,7 @@ __global__ void __launch_bounds__((PHI ? PHI_THREADS : 256), (PHI ? (FAR ? 3 : 4
             const Cic<F> c = cic_setup(q, g.n);
             if (PHI) {
                 F d[3] = {(F)NAN, (F)NAN, (F)NAN};
-                if (ok) fd_read(m0, c, g.n, twocell, d);
+                if (ok) fd_read<typename std::conditional<SHAPE == PHI_ORDERED, uint32_t, int64_t>::type>(m0, c, g.n, twocell, d);
 #pragma unroll
                 for (int a = 0; a < 3; a++) s[a] = (P)d[a];
             } else if (IL) {
@@ -1449,22 +1452,24 @@ int read_shifts_launch(const F* m0, const F* m1, const F* m2, int stride, bool p
     const double ncell = (double)g.n[0] * g.n[1] * g.n[2];
     const double gather_bytes = (double)n * 3 * (sizeof(P) + ob) +
                                 (phi ? std::min(ncell, 32.0 * n) : 3 * std::min(ncell, 8.0 * n)) * sizeof(F);
-#define LAUNCH(O, PH, IL, FAR)                                                                                     \
+#define LAUNCH(O, PH, IL, SHAPE)                                                                                   \
     PRC_LAUNCH_B(PH ? "read_shifts_phi" : "read_shifts_psi", st, gather_bytes,                                     \
-                 read_shifts_kernel<P, F, O, PH, IL, FAR><<<grid, threads, 0, st>>>(m0, m1, m2, g, tc[0], tc[1], tc[2], \
+                 read_shifts_kernel<P, F, O, PH, IL, SHAPE><<<grid, threads, 0, st>>>(m0, m1, m2, g, tc[0], tc[1], tc[2], \
                                                                          (const P*)pos, n, f, los != nullptr, l[0], \
                                                                          l[1], l[2], field, shifted, wrap,          \
                                                                          (O*)out, flags, order,             \
                                                                          (const P*)sorted_pos))
     constexpr bool SINGLE = sizeof(P) == 4 && sizeof(F) == 4;
-    if (phi && (SINGLE || (order == nullptr && ncell * sizeof(F) > PHI_FAR_BYTES))) {
-        if (ob == 4) LAUNCH(float, true, false, true); else LAUNCH(double, true, false, true);
+    if (phi && order == nullptr && (SINGLE || ncell * sizeof(F) > PHI_FAR_BYTES)) {
+        if (ob == 4) LAUNCH(float, true, false, PHI_FAR); else LAUNCH(double, true, false, PHI_FAR);
+    } else if (phi && order == nullptr) {
+        if (ob == 4) LAUNCH(float, true, false, PHI_NEAR); else LAUNCH(double, true, false, PHI_NEAR);
     } else if (phi) {
-        if (ob == 4) LAUNCH(float, true, false, SINGLE); else LAUNCH(double, true, false, SINGLE);
+        if (ob == 4) LAUNCH(float, true, false, PHI_ORDERED); else LAUNCH(double, true, false, PHI_ORDERED);
     } else if (il) {
-        if (ob == 4) LAUNCH(float, false, true, false); else LAUNCH(double, false, true, false);
+        if (ob == 4) LAUNCH(float, false, true, PHI_NEAR); else LAUNCH(double, false, true, PHI_NEAR);
     } else {
-        if (ob == 4) LAUNCH(float, false, false, false); else LAUNCH(double, false, false, false);
+        if (ob == 4) LAUNCH(float, false, false, PHI_NEAR); else LAUNCH(double, false, false, PHI_NEAR);
     }
 #undef LAUNCH
     PRC_CHECK_LAUNCH();
